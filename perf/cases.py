@@ -265,3 +265,34 @@ def tolerance(case):
     # A bf16 step in the tensor that holds a maximum moves a per-tensor scale, and with it the stochastic
     # rounding of part of the gradient's blocks: seen 1e-3 to 0.1 over the gradients of a block.
     return {"rel": 0.03, "max": 0.95}
+
+
+def _dequantized(t):
+    """What quant_nvfp4(t) (round to nearest) stands for, in 64 bits: 1 x 16 blocks along the rows of t, E4M3
+    block scales under one fp32 scale of the tensor, E2M1 codes."""
+    x = t.to(torch.bfloat16).float()
+    blocks = x.view(x.shape[0], -1, 16)
+    top = blocks.abs().amax(-1)
+    six, one = torch.full_like(top, 6.0), x.new_ones(())
+    pts = torch.clamp(top.max(), min=1e-12) / x.new_tensor(2688.0)
+    scale = (top / six / pts).clamp(2.0 ** -6, 448.0).to(torch.float8_e4m3fn).float()
+    v = (blocks * (one / pts / scale)[..., None]).clamp(-6.0, 6.0)
+    a = v.abs()
+    v = torch.where(a < 2, torch.round(v * 2) / 2, torch.where(a < 4, torch.round(v), torch.round(v / 2) * 2))
+    return (v.double() * scale[..., None].double() * pts.double()).view(x.shape)
+
+
+def exact(case, seed):
+    """Products of operands that are rounded to nearest; where an operand is rounded stochastically, or a
+    rounding to bf16 is quantized again, there is no such value."""
+    kind = case["kind"]
+    if kind == "mm" and not case["sr"]:
+        g = _gen(seed)
+        m, n, k = case["m"], case["n"], case["k"]
+        a, b = _normal(g, m, k), _normal(g, k, n)
+        return _dequantized(a) @ _dequantized(b.t().contiguous()).t()
+    if kind == "linear":
+        s = prepare(case, seed)
+        x, w = s["x"].detach(), s["lin"].weight.detach()
+        return [_dequantized(x) @ _dequantized(w).t(), None, None]
+    return None
