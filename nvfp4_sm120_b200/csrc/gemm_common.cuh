@@ -127,6 +127,17 @@ __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sy
 __device__ __forceinline__ uint64_t make_desc_sw128(uint32_t saddr) {
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
+// The same for a 512-byte scale tile (32 rows of 16 bytes, no swizzle: 8-row groups are 128 bytes apart).
+__device__ __forceinline__ uint64_t make_desc_scales(uint32_t saddr) {
+  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(128 >> 4) << 32) | (1ull << 46);
+}
+// One lane of a converged warp.  The tcgen05 instructions take their operands from uniform registers: behind this
+// predicate the compiler knows that one lane runs them, behind `lane == 0` it does not.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+  return p != 0;
+}
 // Instruction descriptor of kind::mxf4nvf4: A/B format E2M1 (code 1), E4M3 scales (0), both K-major,
 // N >> 3 at bit 17, M >> 4 at bit 24, dense K = 64.
 __host__ __device__ constexpr uint32_t make_idesc(int m, int n) {
@@ -377,6 +388,20 @@ inline bool make_operand_map(CUtensorMap* map, const uint8_t* ptr, int64_t rows,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// tiled scale buffer of an operand [rows, k] -> 2-D map of 8-byte words, one row per 128 operand rows; a box is the
+// 2048 contiguous bytes of one K slice in `groups` row groups.  Rows and columns outside read as zero scales.
+inline bool make_scale_map(CUtensorMap* map, const uint8_t* ptr, int64_t rows, int64_t k, int groups) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return false;
+  const cuuint64_t col_tiles = (cuuint64_t)((k / 16 + 3) / 4);
+  cuuint64_t dims[2] = {col_tiles * 64, (cuuint64_t)((rows + 127) / 128)};
+  cuuint64_t strides[1] = {col_tiles * 512};
+  cuuint32_t box[2] = {256u, (cuuint32_t)groups};
+  cuuint32_t estr[2] = {1u, 1u};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<uint8_t*>(ptr), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 // row-major output [M, ldd] -> 2-D tensor map for the epilogue's stores: boxes of 32 rows x 128 bytes
 inline bool make_output_map(CUtensorMap* map, void* d, int64_t M, int64_t N, int64_t ldd, bool f32) {

@@ -2,13 +2,20 @@
 //
 // One cluster of two CTAs per pair of SMs stays resident and walks over 256 x 256 output tiles
 // (tile = cluster index + i * number of clusters, grouped rasterization).  The roles of a CTA:
-//   warp 0      producer: TMA tensor copies of its 128 A rows and its 128 of the 256 B rows
-//               (cta_group::2 form, completing on the leader's barrier; no multicast) and bulk
-//               copies of the scale tiles, into a ring of five stages that runs on across tiles;
-//   warp 1      (leader CTA only) issues tcgen05.mma cta_group::2, M 256 = 128 per CTA, N 256, K 64:
-//               four per K slice, back to back, one barrier wait per slice;
-//   warps 2-5   scale factors shared memory -> registers -> tensor memory (one warp per 32-lane quarter);
-//   warps 6-13  epilogue: tensor memory -> registers -> swizzled shared memory -> TMA store.
+//   warp 0      producer: TMA tensor copies of its 128 A rows, its 128 of the 256 B rows and the scale tiles
+//               of both (cta_group::2 form, all completing on the leader's barrier; no multicast), into a
+//               ring of five stages that runs on across tiles;
+//   warp 1      (leader CTA only) per K slice one barrier wait, then twelve tcgen05.cp (the scale tiles of both CTAs,
+//               shared -> tensor memory) and four tcgen05.mma cta_group::2, M 256 = 128 per CTA, N 256, K 64;
+//   warps 2-9   epilogue: tensor memory -> registers -> swizzled shared memory -> TMA store.
+// What bounds it: the shared-memory data stage (per CTA and slice 304 wavefronts of 128 bytes written by TMA, 256
+// read by the MMAs, 48 by the scale copies, against 512 cycles of tensor work).  The scale copies used to go through
+// registers (four warps each reading all 6 KiB of a slice: 192 wavefronts); tcgen05.cp reads them once.  It pays
+// only when the issuing lane is picked by elect.sync (elect_one): behind `lane == 0` the compiler cannot tell that
+// one lane runs the tcgen05 instructions, every copy then cost about 40 cycles and the kernel 312 us at 8192^3.
+// Measured at 8192^3, bf16 output, one launch after an L2 flush: 223 us through registers, 184 us (5.96 PFLOP/s)
+// this way; 16384 x 4096 x 14336 378 -> 324 us, 4096^3 45 -> 39 us, 4096 x 28672 x 4096 with fp32 output 254 -> 219.
+// Spreading the copies between the MMAs of the slice measured the same.
 // Because the ring never drains, the loads of the next tile are in flight while the epilogue warps
 // empty the accumulator; the MMA issuer only waits for "accumulator read" before the next tile, so
 // the launch, barrier set-up, tensor-memory allocation and pipeline fill are paid once per SM pair,
@@ -32,10 +39,10 @@ constexpr int kSfbBytes = 2 * 4 * 512;
 constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;      // 38912
 constexpr int kOutBytes = 8 * 4096;         // per epilogue warp one box of 32 rows x 128 bytes
 constexpr int kSmemBytes = kStages * kStageBytes + kOutBytes + 1024 + 256;
-constexpr int kSfSets = 1;                  // groups of four scale-factor warps taking the K slices in turn
-constexpr int kEpiWarp0 = 2 + 4 * kSfSets;  // first epilogue warp
+constexpr int kEpiWarp0 = 2;                // first epilogue warp
 constexpr int kThreads = (kEpiWarp0 + 8) * 32;
-constexpr int kSfColsPerStage = 48;
+constexpr int kSfCols = 48;                 // tensor-memory columns of one K slice's scale factors
+constexpr int kSfRing = 4;                  // slices of scale factors in tensor memory
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -62,9 +69,14 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
       " [%0], [%1, {%2, %3}], [%4];"
       ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar_cluster_addr) : "memory");
 }
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-               ::"r"(bar_cluster_addr) : "memory");
+// arrives on the barrier at this offset in both CTAs of the pair
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+// one 512-byte scale tile of each CTA -> four columns of its tensor memory, in all four 32-lane quarters
+__device__ __forceinline__ void tc_copy_scales_pair(uint32_t tmem, uint64_t desc) {
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem), "l"(desc) : "memory");
 }
 __device__ __forceinline__ void tc_mma_nvf4_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                                  uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
@@ -93,7 +105,8 @@ struct TileMap {
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-             const __grid_constant__ CUtensorMap map_d, const Params p) {
+             const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_sfa,
+             const __grid_constant__ CUtensorMap map_sfb, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;                 // same offset in both CTAs of the pair
@@ -102,11 +115,10 @@ gemm3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
   const uint32_t bar_base = base + kStages * kStageBytes + kOutBytes;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };                    // leader: A/B of both CTAs landed
   auto empty_bar = [&](int s) { return bar_base + 8u * (kStages + s); };        // MMAs have read the stage
-  auto sfull_bar = [&](int s) { return bar_base + 8u * (2 * kStages + s); };    // this CTA's scale tiles landed
-  auto sready_bar = [&](int s) { return bar_base + 8u * (3 * kStages + s); };   // leader: scales in TMEM, both CTAs
-  const uint32_t acc_full = bar_base + 8u * (4 * kStages);                      // accumulator complete (both CTAs)
-  const uint32_t acc_empty = bar_base + 8u * (4 * kStages + 1);                 // leader: accumulator read, both CTAs
-  const int misc = kStages * kStageBytes + kOutBytes + 8 * (4 * kStages + 2);
+  const uint32_t acc_full = bar_base + 8u * (2 * kStages);                      // accumulator complete (both CTAs)
+  const uint32_t acc_empty = bar_base + 8u * (2 * kStages + 1);                 // leader: accumulator read, both CTAs
+  const uint32_t never_bar = bar_base + 8u * (2 * kStages + 2);                 // test hook: nothing arrives here
+  const int misc = kStages * kStageBytes + kOutBytes + 8 * (2 * kStages + 3);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + misc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + misc + 8);
 
@@ -117,14 +129,14 @@ gemm3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
   const uint32_t cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1, total = tm.total();
   const int my_tiles = cluster_id < total ? (int)((total - cluster_id + n_clusters - 1) / n_clusters) : 0;
   const int num_kt = (int)((p.K + kTileK - 1) / kTileK);
-  const int64_t sf_col_tiles = (p.K / 16 + 3) / 4;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); mbar_init(sfull_bar(s), 1); mbar_init(sready_bar(s), 8);
+      mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1);
     }
     mbar_init(acc_full, 1);
     mbar_init(acc_empty, 16);
+    mbar_init(never_bar, 1);
     *abort_flag = 0;
     set_wait_limit(abort_flag, p.wait_limit_ns);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -151,140 +163,75 @@ gemm3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         int64_t pair_m0, n0;
         tm.locate(cluster_id + (uint32_t)i * n_clusters, pair_m0, n0);
         const int64_t m0 = pair_m0 + (int64_t)rank * 128;
-        const bool have_sfa = m0 < p.M;                           // padded pair: no such rows in the scale buffer
-        const bool second_sfb = (n0 + 128) < p.N;
-        const uint8_t* sfa_row = p.a_sf + (m0 >> 7) * sf_col_tiles * 512;
-        const uint8_t* sfb_row = p.b_sf + (n0 >> 7) * sf_col_tiles * 512;
         for (int kt = 0; kt < num_kt; ++kt) {
           if (issued >= kStages && !mbar_wait(empty_bar(s), pass ^ 1u, abort_flag)) {
             raise(abort_flag, p.status, kErrProducerWait);
             ok = false;
             break;
           }
-          const int64_t k_left = p.K - (int64_t)kt * kTileK;
-          const int nkb = k_left >= kTileK ? 4 : (int)((k_left + 63) / 64);
-          const uint32_t sf_bytes = (uint32_t)nkb * 512u;
           const uint32_t stage = base + s * kStageBytes;
           const uint32_t leader_full = map_to_cta(full_bar(s), 0);
-          if (leader) mbar_expect_tx(full_bar(s), 2u * (kABytes + kBBytes));
+          if (leader)   // whole boxes always: rows and columns outside the operands arrive as zeros
+            mbar_expect_tx(full_bar(s), 2u * kStageBytes);
           tma_load_2d_pair(stage, &map_a, kt * 128, (int)m0, leader_full);
           tma_load_2d_pair(stage + kABytes, &map_b, kt * 128, (int)(n0 + rank * 128), leader_full);
-          mbar_expect_tx(sfull_bar(s), sf_bytes * ((have_sfa ? 1u : 0u) + 1u + (second_sfb ? 1u : 0u)));
-          const int64_t off = (int64_t)kt * 4 * 512;
-          if (have_sfa) bulk_load(stage + kABytes + kBBytes, sfa_row + off, sf_bytes, sfull_bar(s));
-          bulk_load(stage + kABytes + kBBytes + kSfaBytes, sfb_row + off, sf_bytes, sfull_bar(s));
-          if (second_sfb)
-            bulk_load(stage + kABytes + kBBytes + kSfaBytes + 2048, sfb_row + sf_col_tiles * 512 + off, sf_bytes,
-                      sfull_bar(s));
+          tma_load_2d_pair(stage + kABytes + kBBytes, &map_sfa, kt * 256, (int)(m0 >> 7), leader_full);
+          tma_load_2d_pair(stage + kABytes + kBBytes + kSfaBytes, &map_sfb, kt * 256, (int)(n0 >> 7), leader_full);
           ++issued;
           if (++s == kStages) { s = 0; pass ^= 1u; }
         }
       }
       if (*abort_flag != 0) {
         // give copies already in flight a bounded chance to land before shared memory goes away
+        // (the leader's barriers count the copies of both CTAs)
         const int first_g = issued > kStages ? issued - kStages : 0;
-        for (int g = first_g; g < issued; ++g) {
-          for (uint32_t n = 0; n < (1u << 16) && !mbar_try_wait(sfull_bar(g % kStages), (g / kStages) & 1); ++n) {}
-          if (leader)
-            for (uint32_t n = 0; n < (1u << 16) && !mbar_try_wait(full_bar(g % kStages), (g / kStages) & 1); ++n) {}
-        }
+        for (int g = first_g; leader && g < issued; ++g)
+          for (uint32_t n = 0; n < (1u << 16) && !mbar_try_wait(full_bar(g % kStages), (g / kStages) & 1); ++n) {}
+        if (!leader) __nanosleep(50000);
       }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA only) ------------------------------
-    if (lane == 0 && leader) {
+    if (leader) {
       constexpr uint32_t idesc = make_idesc(256, kTileN);
       const int whole_kt = (int)min((int64_t)num_kt, p.K / kTileK);     // K slices with all four K=64 blocks
-      const uint32_t partner_empty0 = map_to_cta(empty_bar(0), 1);
-      const uint32_t partner_acc_full = map_to_cta(acc_full, 1);
       int s = 0;
-      uint32_t par = 0;
+      uint32_t par = 0, sf = 0;
       bool ok = true;
       for (int i = 0; i < my_tiles && ok; ++i) {
         if (i > 0) {                                            // the epilogue warps have read the accumulator
-          if (!mbar_wait(acc_empty, (uint32_t)(i - 1) & 1u, abort_flag)) {
-            raise(abort_flag, p.status, kErrMmaWait);
-            break;
-          }
+          ok = __all_sync(0xffffffffu, mbar_wait(acc_empty, (uint32_t)(i - 1) & 1u, abort_flag));
+          if (!ok) { raise(abort_flag, p.status, kErrMmaWait); break; }
           tc_fence_after();
         }
         for (int kt = 0; kt < num_kt; ++kt) {
-          // one wait per K slice: the leader's scale warps arrive only after the operand tiles of both
-          // CTAs have landed, so "scales ready" covers "data landed"
-          if (!mbar_wait(sready_bar(s), par, abort_flag)) {
-            raise(abort_flag, p.status, kErrMmaWait);
-            ok = false;
-            break;
-          }
+          ok = __all_sync(0xffffffffu, mbar_wait(p.drop_first_scale_arrival ? never_bar : full_bar(s), par, abort_flag));
+          if (!ok) { raise(abort_flag, p.status, kErrMmaWait); break; }
           tc_fence_after();
           const uint32_t stage = base + s * kStageBytes;
-          const uint32_t t_sfa = tmem_sf0 + s * kSfColsPerStage, t_sfb = t_sfa + 16;
+          const uint32_t t_sfa = tmem_sf0 + sf * kSfCols, t_sfb = t_sfa + 16;
           const uint64_t da = make_desc_sw128(stage), db = make_desc_sw128(stage + kABytes);
-          if (kt < whole_kt) {                                  // back to back, nothing in between
-            tc_mma_nvf4_pair(tmem_base, da, db, idesc, t_sfa, t_sfb, kt > 0 ? 1u : 0u);
-            tc_mma_nvf4_pair(tmem_base, da + 2u, db + 2u, idesc, t_sfa + 4, t_sfb + 8, 1u);
-            tc_mma_nvf4_pair(tmem_base, da + 4u, db + 4u, idesc, t_sfa + 8, t_sfb + 16, 1u);
-            tc_mma_nvf4_pair(tmem_base, da + 6u, db + 6u, idesc, t_sfa + 12, t_sfb + 24, 1u);
-          } else {
-            const int nkb = (int)((p.K - (int64_t)kt * kTileK + 63) / 64);
-            for (int kb = 0; kb < nkb; ++kb)
-              tc_mma_nvf4_pair(tmem_base, da + 2u * kb, db + 2u * kb, idesc, t_sfa + 4 * kb, t_sfb + 8 * kb,
-                               (kt > 0 || kb > 0) ? 1u : 0u);
+          const uint64_t dsa = make_desc_scales(stage + kABytes + kBBytes), dsb = dsa + (kSfaBytes >> 4);
+          const int nkb = kt < whole_kt ? 4 : (int)((p.K - (int64_t)kt * kTileK + 63) / 64);
+          if (elect_one()) {
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb) {
+              tc_copy_scales_pair(t_sfa + 4 * kb, dsa + 32u * kb);
+              tc_copy_scales_pair(t_sfb + 8 * kb, dsb + 32u * kb);
+              tc_copy_scales_pair(t_sfb + 8 * kb + 4, dsb + 128u + 32u * kb);
+            }
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb)
+              if (kb < nkb)
+                tc_mma_nvf4_pair(tmem_base, da + 2u * kb, db + 2u * kb, idesc, t_sfa + 4 * kb, t_sfb + 8 * kb,
+                                 (kt > 0 || kb > 0) ? 1u : 0u);
+            tc_commit_pair(empty_bar(s));
+            if (kt == num_kt - 1) tc_commit_pair(acc_full);
           }
-          tc_commit_pair(empty_bar(s));                       // frees the stage here ...
-          tc_commit_pair(partner_empty0 + 8u * s);            // ... and in the partner CTA
+          __syncwarp();
           if (++s == kStages) { s = 0; par ^= 1u; }
+          if (++sf == kSfRing) sf = 0;
         }
-        if (ok) {
-          tc_commit_pair(acc_full);
-          tc_commit_pair(partner_acc_full);
-        }
-      }
-    }
-  } else if (warp < kEpiWarp0) {
-    // ------------------------------ scale factors ------------------------------
-    // Lane l / 32-bit column c of a K=64 block must hold, in every 32-lane quarter of tensor memory,
-    // the four E4M3 scales of row 32c + l: exactly 16 bytes per lane of the 512-byte tile the
-    // quantizer wrote, so one 128-bit shared load per tile and lane feeds four columns, and each
-    // warp writes the copy of its own quarter.  The two sets take alternate K slices.
-    const int quad = warp & 3;
-    const int set = (warp - 2) >> 2;
-    const uint32_t leader_ready0 = map_to_cta(sready_bar(0), 0);
-    const int64_t total_g = (int64_t)my_tiles * num_kt;
-    bool ok = true;
-    for (int64_t g = set; g < total_g && ok; g += kSfSets) {
-      const int s = (int)(g % kStages);
-      const uint32_t par = (uint32_t)(g / kStages) & 1u;
-      if (lane == 0) {
-        ok = mbar_wait(sfull_bar(s), par, abort_flag);
-        if (ok && leader) ok = mbar_wait(full_bar(s), par, abort_flag);   // see the MMA issuer
-      }
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      if (!ok) { if (lane == 0) raise(abort_flag, p.status, kErrScaleWait); break; }
-      const uint8_t* sf_s = smem + s * kStageBytes + kABytes + kBBytes + lane * 16;
-      const uint32_t t_sf = tmem_sf0 + s * kSfColsPerStage + ((uint32_t)(quad * 32) << 16);
-      uint32_t r[16];
-#pragma unroll
-      for (int kb = 0; kb < 4; ++kb) {
-        const uint4 v = *reinterpret_cast<const uint4*>(sf_s + 512 * kb);
-        r[4 * kb] = v.x; r[4 * kb + 1] = v.y; r[4 * kb + 2] = v.z; r[4 * kb + 3] = v.w;
-      }
-      tc_st_32x32b_x16(t_sf, r);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int kb = 2 * half + (q >> 1), tile = q & 1;
-          const uint4 v = *reinterpret_cast<const uint4*>(sf_s + kSfaBytes + 2048 * tile + 512 * kb);
-          r[4 * q] = v.x; r[4 * q + 1] = v.y; r[4 * q + 2] = v.z; r[4 * q + 3] = v.w;
-        }
-        tc_st_32x32b_x16(t_sf + 16 + 16 * half, r);
-      }
-      tc_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0 && !(p.drop_first_scale_arrival && g == 0)) {
-        if (leader) mbar_arrive(sready_bar(s)); else mbar_arrive_cluster(leader_ready0 + 8u * s);
       }
     }
   } else {
@@ -397,6 +344,9 @@ gemm3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
 
 int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_d, const Params& p,
                 cudaStream_t stream) {
+  CUtensorMap map_sfa, map_sfb;
+  if (!make_scale_map(&map_sfa, p.a_sf, p.M, p.K, 1) || !make_scale_map(&map_sfb, p.b_sf, p.N, p.K, 2))
+    return NVFP4_E_DRIVER;
   static std::atomic<int> sm_count[64];         // 0 = not looked up yet; a second look-up is harmless
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return NVFP4_E_LAUNCH;
@@ -411,7 +361,7 @@ int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtens
   const int64_t tiles = ((p.N + kTileN - 1) / kTileN) * ((p.M + 255) / 256);
   if (tiles > 0x3fffffffLL) return NVFP4_E_SHAPE;
   const int64_t clusters = tiles < sms / 2 ? tiles : sms / 2;    // one resident pair per two SMs
-  gemm3_kernel<<<dim3((unsigned)(2 * clusters)), kThreads, kSmemBytes, stream>>>(map_a, map_b, map_d, p);
+  gemm3_kernel<<<dim3((unsigned)(2 * clusters)), kThreads, kSmemBytes, stream>>>(map_a, map_b, map_d, map_sfa, map_sfb, p);
   return cudaGetLastError() == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
 }
 
