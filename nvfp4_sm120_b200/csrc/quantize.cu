@@ -300,74 +300,6 @@ __global__ void __launch_bounds__(256) amax_rht_cols_kernel(const uint16_t* __re
   cta_max_to(amax, m);
 }
 
-template <bool SR, bool RHT>
-__global__ void __launch_bounds__(256) quant_cols_kernel(const uint16_t* __restrict__ x, int64_t rows,
-                                                         int64_t cols, int64_t ld,
-                                                         const float* __restrict__ signs16,
-                                                         const float* __restrict__ amax,
-                                                         const PhiloxKeys keys, uint64_t offset,
-                                                         uint8_t* __restrict__ qdata,
-                                                         uint8_t* __restrict__ scales,
-                                                         float* __restrict__ pts_out,
-                                                         uint64_t ctr_pitch, uint64_t ctr_base) {
-  // Philox counter of output block (column c, row block kb) = c * ctr_pitch + ctr_base + kb
-  __shared__ float recip_tab[128];
-  const GlobalScale g = global_scale(amax, recip_tab);
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && pts_out != nullptr) *pts_out = g.pts;
-  uint32_t sm[16];
-  if (RHT) {
-    float sg[16];
-    load_signs(signs16, sg);
-    sign_masks(sg, sm);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) sm[i] = 0u;
-  }
-  const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
-  if (c >= cols) return;
-  const int64_t r_base = (int64_t)blockIdx.y * 64;
-  const int64_t blk_per_orow = rows >> 4;            // blocks per OUTPUT row (K = rows)
-  const int64_t col_tiles = (blk_per_orow + 3) >> 2;
-  const int64_t out_ld = rows >> 1;                  // bytes per output row
-  uint32_t q[2][8];
-  uint32_t sfw[2] = {0u, 0u};
-  int nvalid = 0;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int64_t r0 = r_base + 16 * j;
-    if (r0 < rows) {
-      float v0[16], v1[16];
-      load_col_pair_block<RHT>(x, ld, r0, c, sm, v0, v1);
-      const uint64_t kb = (uint64_t)(r0 >> 4);
-      uint32_t sf0, sf1;
-      encode_block<SR>(v0, g, (uint64_t)c * ctr_pitch + ctr_base + kb, keys, offset, q[0][2 * j], q[0][2 * j + 1], sf0);
-      encode_block<SR>(v1, g, (uint64_t)(c + 1) * ctr_pitch + ctr_base + kb, keys, offset, q[1][2 * j], q[1][2 * j + 1], sf1);
-      sfw[0] |= sf0 << (8 * j);
-      sfw[1] |= sf1 << (8 * j);
-      nvalid = j + 1;
-    }
-  }
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    uint8_t* orow = qdata + (c + h) * out_ld + (r_base >> 1);
-    const size_t so = sf_offset(c + h, r_base >> 4, col_tiles);
-    if (nvalid == 4 && (out_ld & 15) == 0) {
-      reinterpret_cast<uint4*>(orow)[0] = make_uint4(q[h][0], q[h][1], q[h][2], q[h][3]);
-      reinterpret_cast<uint4*>(orow)[1] = make_uint4(q[h][4], q[h][5], q[h][6], q[h][7]);
-      *reinterpret_cast<uint32_t*>(scales + so) = sfw[h];
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (j < nvalid) {
-          *reinterpret_cast<uint2*>(orow + 8 * j) = make_uint2(q[h][2 * j], q[h][2 * j + 1]);
-          scales[so + j] = (uint8_t)(sfw[h] >> (8 * j));
-        }
-      }
-    }
-  }
-}
-
-
 // ---------------------------------------------------------------------------------------
 // Wide form of the column MAXIMUM kernels for 16-byte rows (cols % 8 == 0).  The narrow kernels above read
 // 128 contiguous bytes of a row per warp instruction; here a CTA takes tiles of 16 rows x 512 columns
@@ -465,20 +397,18 @@ __global__ void __launch_bounds__(256) amax_cols_wide_kernel(const uint16_t* __r
 }
 
 // ---------------------------------------------------------------------------------------
-// weights: both layouts from one read.  A CTA takes a 64 x 64 tile of w [rows, cols]; thread
+// weights under 16 x 16 scaling: both layouts from one read.  A CTA takes a 64 x 64 tile of w [rows, cols]; thread
 // (row t / 4, segment t % 4) loads the 16 elements of row-wise block (row, segment) and leaves them in
 // a padded shared tile, from which thread (column t % 64, row block t / 64) reads the 16 elements of
-// column-wise block (column, row block).  Round to nearest only (weights).  TWO_D: one scale per
-// 16 x 16 tile, shared by the row-wise and the column-wise blocks that cross it, so that both
-// quantized layouts hold the same values (the reference simulator's weight scaling,
-// nvfp4_validate.py:68-82); otherwise every block has its own 1 x 16 scale, as quant_nvfp4 gives.
+// column-wise block (column, row block).  Round to nearest.  One scale per 16 x 16 tile is shared by the row-wise and
+// the column-wise blocks that cross it, so that both quantized layouts hold the same values (the reference
+// simulator's weight scaling, nvfp4_validate.py:68-82).  1 x 16 scaling is quantize_dual.cu.
 // ---------------------------------------------------------------------------------------
-template <bool TWO_D>
-__global__ void __launch_bounds__(256) quant_weight_dual_kernel(const uint16_t* __restrict__ w, int64_t rows, int64_t cols,
-                                                                int64_t ld, const float* __restrict__ amax,
-                                                                uint8_t* __restrict__ q_rows, uint8_t* __restrict__ sf_rows,
-                                                                uint8_t* __restrict__ q_cols, uint8_t* __restrict__ sf_cols,
-                                                                float* __restrict__ pts_out) {
+__global__ void __launch_bounds__(256) quant_weight_2d_kernel(const uint16_t* __restrict__ w, int64_t rows, int64_t cols,
+                                                              int64_t ld, const float* __restrict__ amax,
+                                                              uint8_t* __restrict__ q_rows, uint8_t* __restrict__ sf_rows,
+                                                              uint8_t* __restrict__ q_cols, uint8_t* __restrict__ sf_cols,
+                                                              float* __restrict__ pts_out) {
   __shared__ uint16_t tile[64][66];          // 33 words per row: a column walk touches 16 different banks
   __shared__ float bmax[64][4];              // row-wise block maxima of the tile
   __shared__ float tmax[4][4];               // 16 x 16 tile maxima
@@ -505,23 +435,20 @@ __global__ void __launch_bounds__(256) quant_weight_dual_kernel(const uint16_t* 
     v[2 * j + 1] = bf16_hi(wv[j]);
     *reinterpret_cast<uint32_t*>(&tile[r][seg * 16 + 2 * j]) = wv[j];
   }
-  const float my_max = block_amax16(v);
-  if (TWO_D) bmax[r][seg] = my_max;
+  bmax[r][seg] = block_amax16(v);
   __syncthreads();
-  if (TWO_D) {
-    if (t < 16) {
-      const int rb = t >> 2, cb = t & 3;
-      float m = 0.0f;
+  if (t < 16) {
+    const int rb = t >> 2, cb = t & 3;
+    float m = 0.0f;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) m = fmaxf(m, bmax[rb * 16 + i][cb]);
-      tmax[rb][cb] = m;
-    }
-    __syncthreads();
+    for (int i = 0; i < 16; ++i) m = fmaxf(m, bmax[rb * 16 + i][cb]);
+    tmax[rb][cb] = m;
   }
+  __syncthreads();
   // ---- row-wise output ----
   if (have) {
     uint32_t lo, hi, sf;
-    encode_block_scaled<false>(v, TWO_D ? tmax[r >> 4][seg] : my_max, g, 0, keys, 0, lo, hi, sf);
+    encode_block_scaled<false>(v, tmax[r >> 4][seg], g, 0, keys, 0, lo, hi, sf);
     const int64_t kb = gc >> 4;
     *reinterpret_cast<uint2*>(q_rows + gr * (cols >> 1) + kb * 8) = make_uint2(lo, hi);
     sf_rows[sf_offset(gr, kb, ((cols >> 4) + 3) >> 2)] = (uint8_t)sf;
@@ -534,87 +461,13 @@ __global__ void __launch_bounds__(256) quant_weight_dual_kernel(const uint16_t* 
 #pragma unroll
     for (int i = 0; i < 16; ++i) u[i] = __uint_as_float((uint32_t)tile[rb * 16 + i][c] << 16);
     uint32_t lo, hi, sf;
-    encode_block_scaled<false>(u, TWO_D ? tmax[rb][c >> 4] : block_amax16(u), g, 0, keys, 0, lo, hi, sf);
+    encode_block_scaled<false>(u, tmax[rb][c >> 4], g, 0, keys, 0, lo, hi, sf);
     const int64_t kb = orow0 >> 4;
     *reinterpret_cast<uint2*>(q_cols + oc * (rows >> 1) + kb * 8) = make_uint2(lo, hi);
     sf_cols[sf_offset(oc, kb, ((rows >> 4) + 3) >> 2)] = (uint8_t)sf;
   }
 }
 
-
-// ---------------------------------------------------------------------------------------
-// activations and gradients: both layouts from one read.  Every operand of FP4Linear is needed
-// twice: x row-wise for fprop and x^T (Hadamard along the tokens) for wgrad, dY row-wise
-// (stochastic) for dgrad and dY^T (Hadamard + stochastic) for wgrad (nvfp4_train.py:36-55).  Same
-// 64 x 64 tiling as the weight kernel above: thread (row t / 4, segment t % 4) encodes row-wise
-// block (row, segment) with the plain maximum, then thread (column t % 64, row block t / 64) reads
-// its 16 rows of one column from the shared tile, applies the random-sign Hadamard along the rows
-// and encodes the column-wise block with the maximum of the transformed tensor.  Each layout has
-// its own per-tensor maximum, seed and Philox counter (counter of a block = its index in the whole
-// tensor of that layout: out_row * pitch + base + k_block), so the bytes are those of the two
-// separate quantizations.
-// ---------------------------------------------------------------------------------------
-struct DualCounters { uint64_t pitch_r, base_r, pitch_c, base_c; };
-
-template <bool SR_R, bool SR_C>
-__global__ void __launch_bounds__(256) quant_act_dual_kernel(const uint16_t* __restrict__ x, int64_t rows, int64_t cols,
-                                                             int64_t ld, const float* __restrict__ signs16,
-                                                             const float* __restrict__ amax_r,
-                                                             const float* __restrict__ amax_c, const PhiloxKeys keys_r,
-                                                             const PhiloxKeys keys_c, uint64_t offset, DualCounters ctr,
-                                                             uint8_t* __restrict__ q_rows, uint8_t* __restrict__ sf_rows,
-                                                             float* __restrict__ pts_r, uint8_t* __restrict__ q_cols,
-                                                             uint8_t* __restrict__ sf_cols, float* __restrict__ pts_c) {
-  __shared__ uint16_t tile[64][66];          // 33 words per row: a column walk touches 16 different banks
-  __shared__ float recip_r[128], recip_c[128];
-  const GlobalScale g_r = global_scale(amax_r, recip_r), g_c = global_scale(amax_c, recip_c);
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
-    if (pts_r != nullptr) *pts_r = g_r.pts;
-    if (pts_c != nullptr) *pts_c = g_c.pts;
-  }
-  const int t = threadIdx.x;
-  const int64_t r0 = (int64_t)blockIdx.y * 64, c0 = (int64_t)blockIdx.x * 64;
-  const int r = t >> 2, seg = t & 3;
-  const int64_t gr = r0 + r, gc = c0 + seg * 16;
-  const bool have = gr < rows && gc < cols;          // rows and cols are multiples of 16: a block is whole or absent
-  uint32_t wv[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-  if (have) {
-    const uint4* p = reinterpret_cast<const uint4*>(x + gr * ld + gc);
-    const uint4 a = __ldg(p), b = __ldg(p + 1);
-    wv[0] = a.x; wv[1] = a.y; wv[2] = a.z; wv[3] = a.w; wv[4] = b.x; wv[5] = b.y; wv[6] = b.z; wv[7] = b.w;
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) *reinterpret_cast<uint32_t*>(&tile[r][seg * 16 + 2 * j]) = wv[j];
-  if (have) {
-    float v[16];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      v[2 * j] = bf16_lo(wv[j]);
-      v[2 * j + 1] = bf16_hi(wv[j]);
-    }
-    uint32_t lo, hi, sf;
-    const int64_t kb = gc >> 4;
-    encode_block<SR_R>(v, g_r, (uint64_t)gr * ctr.pitch_r + ctr.base_r + (uint64_t)kb, keys_r, offset, lo, hi, sf);
-    *reinterpret_cast<uint2*>(q_rows + gr * (cols >> 1) + kb * 8) = make_uint2(lo, hi);
-    sf_rows[sf_offset(gr, kb, ((cols >> 4) + 3) >> 2)] = (uint8_t)sf;
-  }
-  __syncthreads();
-  const int c = t & 63, rb = t >> 6;
-  const int64_t oc = c0 + c, orow0 = r0 + rb * 16;
-  if (oc < cols && orow0 < rows) {
-    float sg[16];
-    load_signs(signs16, sg);
-    float u[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) u[i] = __uint_as_float((uint32_t)tile[rb * 16 + i][c] << 16) * sg[i];
-    hadamard16_inplace(u);
-    uint32_t lo, hi, sf;
-    const int64_t kb = orow0 >> 4;
-    encode_block<SR_C>(u, g_c, (uint64_t)oc * ctr.pitch_c + ctr.base_c + (uint64_t)kb, keys_c, offset, lo, hi, sf);
-    *reinterpret_cast<uint2*>(q_cols + oc * (rows >> 1) + kb * 8) = make_uint2(lo, hi);
-    sf_cols[sf_offset(oc, kb, ((rows >> 4) + 3) >> 2)] = (uint8_t)sf;
-  }
-}
 
 // plain maximum and maximum after the Hadamard transform along the rows, from one read
 __global__ void __launch_bounds__(256) amax_both_cols_kernel(const uint16_t* __restrict__ x, int64_t rows,
@@ -698,6 +551,12 @@ extern "C" int nvfp4_amax_bf16(const void* x, int64_t rows, int64_t cols, int64_
   return cudaGetLastError() == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
 }
 
+namespace nvfp4 { namespace dual {
+int launch(const void* x, int64_t rows, int64_t cols, int64_t ld, int rows_mode, bool sr_c, const float* signs16,
+           const float* amax_r, const float* amax_c, uint64_t seed_r, uint64_t seed_c, uint64_t offset,
+           const uint64_t* counters4, uint8_t* q_r, uint8_t* sf_r, float* pts_r, uint8_t* q_c, uint8_t* sf_c, float* pts_c,
+           cudaStream_t stream);
+}}
 namespace nvfp4 { namespace fused {
 int quantize_rows_known_amax(const void* x, int64_t rows, int64_t cols, int64_t ld, int mode, int rht,
                              const float* signs16, const float* amax, uint64_t seed, uint64_t offset,
@@ -717,46 +576,36 @@ extern "C" int nvfp4_quantize_shard_bf16(const void* x, int64_t rows, int64_t co
   if (!aligned16(x) || (ld & 7) != 0 || (reinterpret_cast<uintptr_t>(qdata) & 15u) != 0 ||
       (reinterpret_cast<uintptr_t>(scales) & 15u) != 0 || (rht && !aligned16(signs16)))
     return NVFP4_E_ALIGN;
-  const int64_t out_rows = transpose ? cols : rows;
-  const int64_t k = transpose ? rows : cols;
-  if ((k & 15) != 0) return NVFP4_E_SHAPE;
+  if (((transpose ? rows : cols) & 15) != 0) return NVFP4_E_SHAPE;
   if (transpose && (cols & 1) != 0) return NVFP4_E_SHAPE;
-  if (!transpose) {
-    // row-wise output with the maximum given: one streaming pass of the single-launch kernel's
-    // quantize phase (it declines only tensors of 2^31 blocks or more, which the plain kernel takes)
-    const int rc = nvfp4::fused::quantize_rows_known_amax(x, rows, cols, ld, mode, rht, signs16, amax, seed, offset,
-                                                          counter_pitch, counter_base, qdata, scales, pts_out, stream);
-    if (rc != NVFP4_E_LIMIT) return rc;
+  const bool sr = mode == NVFP4_ROUND_STOCHASTIC;
+  if (transpose) {
+    if ((rows + 63) / 64 > 65535) return NVFP4_E_SHAPE;
+    const uint64_t ctr[4] = {0, 0, counter_pitch, counter_base};
+    return nvfp4::dual::launch(x, rows, cols, ld, 0, sr, rht ? signs16 : nullptr, nullptr, amax, 0, seed, offset, ctr,
+                               nullptr, nullptr, nullptr, qdata, scales, pts_out, stream);
   }
+  // row-wise output with the maximum given: one streaming pass of the single-launch kernel's
+  // quantize phase (it declines only tensors of 2^31 blocks or more, which the plain kernel takes)
+  const int rc = nvfp4::fused::quantize_rows_known_amax(x, rows, cols, ld, mode, rht, signs16, amax, seed, offset,
+                                                        counter_pitch, counter_base, qdata, scales, pts_out, stream);
+  if (rc != NVFP4_E_LIMIT) return rc;
   // padding of the tiled scale buffer must read as zero (the reference pads with zeros)
-  const int64_t sm = (out_rows + 127) / 128 * 128, sk = (k / 16 + 3) / 4 * 4;
-  if (sm != out_rows || sk != k / 16) {
+  const int64_t sm = (rows + 127) / 128 * 128, sk = (cols / 16 + 3) / 4 * 4;
+  if (sm != rows || sk != cols / 16) {
     if (cudaMemsetAsync(scales, 0, (size_t)(sm * sk), stream) != cudaSuccess) return NVFP4_E_LAUNCH;
   }
   const uint16_t* xp = static_cast<const uint16_t*>(x);
-  const bool sr = mode == NVFP4_ROUND_STOCHASTIC;
   const PhiloxKeys keys = make_philox_keys(seed);
-  if (!transpose) {
-    const int bpr = (int)(cols >> 4);
-    const int grid = grid_for(rows * bpr, 256, 1 << 30);
+  const int bpr = (int)(cols >> 4);
+  const int grid = grid_for(rows * bpr, 256, 1 << 30);
 #define NVFP4_LAUNCH_ROWS(SR_, RHT_) \
-    quant_rows_kernel<SR_, RHT_><<<grid, 256, 0, stream>>>(xp, rows, bpr, ld, signs16, amax, keys, offset, qdata, scales, pts_out, counter_pitch, counter_base)
-    if (sr && rht) NVFP4_LAUNCH_ROWS(true, true);
-    else if (sr) NVFP4_LAUNCH_ROWS(true, false);
-    else if (rht) NVFP4_LAUNCH_ROWS(false, true);
-    else NVFP4_LAUNCH_ROWS(false, false);
+  quant_rows_kernel<SR_, RHT_><<<grid, 256, 0, stream>>>(xp, rows, bpr, ld, signs16, amax, keys, offset, qdata, scales, pts_out, counter_pitch, counter_base)
+  if (sr && rht) NVFP4_LAUNCH_ROWS(true, true);
+  else if (sr) NVFP4_LAUNCH_ROWS(true, false);
+  else if (rht) NVFP4_LAUNCH_ROWS(false, true);
+  else NVFP4_LAUNCH_ROWS(false, false);
 #undef NVFP4_LAUNCH_ROWS
-  } else {
-    dim3 grid((unsigned)((cols / 2 + 255) / 256), (unsigned)((rows + 63) / 64));
-    if (grid.y > 65535u) return NVFP4_E_SHAPE;
-#define NVFP4_LAUNCH_COLS(SR_, RHT_) \
-    quant_cols_kernel<SR_, RHT_><<<grid, 256, 0, stream>>>(xp, rows, cols, ld, signs16, amax, keys, offset, qdata, scales, pts_out, counter_pitch, counter_base)
-    if (sr && rht) NVFP4_LAUNCH_COLS(true, true);
-    else if (sr) NVFP4_LAUNCH_COLS(true, false);
-    else if (rht) NVFP4_LAUNCH_COLS(false, true);
-    else NVFP4_LAUNCH_COLS(false, false);
-#undef NVFP4_LAUNCH_COLS
-  }
   return cudaGetLastError() == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
 }
 
@@ -770,6 +619,12 @@ extern "C" int nvfp4_quantize_weight_bf16(const void* w, int64_t rows, int64_t c
   if (!aligned16(w) || (ld & 7) != 0 || !aligned16(qdata_rows) || !aligned16(qdata_cols) || !aligned16(scales_rows) ||
       !aligned16(scales_cols))
     return NVFP4_E_ALIGN;
+  if ((rows + 63) / 64 > 65535) return NVFP4_E_LIMIT;
+  if (!two_d) {
+    const uint64_t ctr[4] = {0, 0, 0, 0};                       // round to nearest: unused
+    return nvfp4::dual::launch(w, rows, cols, ld, 1, false, nullptr, amax, amax, 0, 0, 0, ctr, qdata_rows, scales_rows,
+                               pts_out, qdata_cols, scales_cols, nullptr, stream);
+  }
   // padding of the tiled scale buffers must read as zero
   auto clear_if_padded = [&](uint8_t* sf, int64_t m, int64_t k) {
     const int64_t sm = (m + 127) / 128 * 128, sk = (k / 16 + 3) / 4 * 4;
@@ -778,14 +633,8 @@ extern "C" int nvfp4_quantize_weight_bf16(const void* w, int64_t rows, int64_t c
   };
   if (!clear_if_padded(scales_rows, rows, cols) || !clear_if_padded(scales_cols, cols, rows)) return NVFP4_E_LAUNCH;
   const dim3 grid((unsigned)((cols + 63) / 64), (unsigned)((rows + 63) / 64));
-  if (grid.y > 65535u) return NVFP4_E_LIMIT;
-  const uint16_t* wp = static_cast<const uint16_t*>(w);
-  if (two_d)
-    quant_weight_dual_kernel<true><<<grid, 256, 0, stream>>>(wp, rows, cols, ld, amax, qdata_rows, scales_rows, qdata_cols,
-                                                             scales_cols, pts_out);
-  else
-    quant_weight_dual_kernel<false><<<grid, 256, 0, stream>>>(wp, rows, cols, ld, amax, qdata_rows, scales_rows, qdata_cols,
-                                                              scales_cols, pts_out);
+  quant_weight_2d_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(w), rows, cols, ld, amax, qdata_rows,
+                                                   scales_rows, qdata_cols, scales_cols, pts_out);
   return cudaGetLastError() == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
 }
 
@@ -823,32 +672,17 @@ extern "C" int nvfp4_quantize_dual_bf16(const void* x, int64_t rows, int64_t col
   if (!aligned16(x) || (ld & 7) != 0 || !aligned16(qdata_rows) || !aligned16(qdata_cols) || !aligned16(scales_rows) ||
       !aligned16(scales_cols) || !aligned16(signs16))
     return NVFP4_E_ALIGN;
-  DualCounters ctr{(uint64_t)(cols >> 4), 0, (uint64_t)(rows >> 4), 0};      // the tensor is whole
-  if (counters4 != nullptr) ctr = DualCounters{counters4[0], counters4[1], counters4[2], counters4[3]};
+  uint64_t ctr[4] = {(uint64_t)(cols >> 4), 0, (uint64_t)(rows >> 4), 0};      // pitch, base of rows / cols: a whole tensor
+  if (counters4 != nullptr)
+    for (int i = 0; i < 4; ++i) ctr[i] = counters4[i];
   // the hardware draws from a 32-bit counter word pair; keep both layouts' counters inside 2^64 trivially,
   // and inside the documented 2^32 blocks per tensor
-  if ((uint64_t)rows * ctr.pitch_r + ctr.base_r >= (1ull << 32) || (uint64_t)cols * ctr.pitch_c + ctr.base_c >= (1ull << 32))
+  if ((uint64_t)rows * ctr[0] + ctr[1] >= (1ull << 32) || (uint64_t)cols * ctr[2] + ctr[3] >= (1ull << 32))
     return NVFP4_E_LIMIT;
-  auto clear_if_padded = [&](uint8_t* sf, int64_t m, int64_t k) {
-    const int64_t sm = (m + 127) / 128 * 128, sk = (k / 16 + 3) / 4 * 4;
-    if (sm == m && sk == k / 16) return true;
-    return cudaMemsetAsync(sf, 0, (size_t)(sm * sk), stream) == cudaSuccess;
-  };
-  if (!clear_if_padded(scales_rows, rows, cols) || !clear_if_padded(scales_cols, cols, rows)) return NVFP4_E_LAUNCH;
-  const dim3 grid((unsigned)((cols + 63) / 64), (unsigned)((rows + 63) / 64));
-  if (grid.y > 65535u) return NVFP4_E_LIMIT;
-  const uint16_t* xp = static_cast<const uint16_t*>(x);
-  const bool sr_r = mode_rows == NVFP4_ROUND_STOCHASTIC, sr_c = mode_cols == NVFP4_ROUND_STOCHASTIC;
-  const PhiloxKeys keys_r = make_philox_keys(seed_rows), keys_c = make_philox_keys(seed_cols);
-#define NVFP4_LAUNCH_DUAL(R_, C_) \
-  quant_act_dual_kernel<R_, C_><<<grid, 256, 0, stream>>>(xp, rows, cols, ld, signs16, amax_rows, amax_cols, keys_r, \
-      keys_c, offset, ctr, qdata_rows, scales_rows, pts_rows, qdata_cols, scales_cols, pts_cols)
-  if (sr_r && sr_c) NVFP4_LAUNCH_DUAL(true, true);
-  else if (sr_r) NVFP4_LAUNCH_DUAL(true, false);
-  else if (sr_c) NVFP4_LAUNCH_DUAL(false, true);
-  else NVFP4_LAUNCH_DUAL(false, false);
-#undef NVFP4_LAUNCH_DUAL
-  return cudaGetLastError() == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
+  if ((rows + 63) / 64 > 65535) return NVFP4_E_LIMIT;
+  return nvfp4::dual::launch(x, rows, cols, ld, mode_rows == NVFP4_ROUND_STOCHASTIC ? 2 : 1,
+                             mode_cols == NVFP4_ROUND_STOCHASTIC, signs16, amax_rows, amax_cols, seed_rows, seed_cols,
+                             offset, ctr, qdata_rows, scales_rows, pts_rows, qdata_cols, scales_cols, pts_cols, stream);
 }
 
 extern "C" int nvfp4_quantize_bf16(const void* x, int64_t rows, int64_t cols, int64_t ld, int transpose,

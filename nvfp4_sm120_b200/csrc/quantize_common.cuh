@@ -74,6 +74,19 @@ __device__ __forceinline__ float amax_packed8(const uint32_t (&w)[8]) {
   return __uint_as_float(max(m << 16, m & 0xffff0000u));
 }
 
+// max(m, |a|, |b|) as one three-input instruction (a NaN operand does not count, as with fmaxf)
+__device__ __forceinline__ float max3_abs(float m, float a, float b) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(fabsf(a)), "f"(fabsf(b)));
+  return r;
+}
+__device__ __forceinline__ float max_abs16(const float (&v)[16]) {
+  float a = 0.0f, b = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 16; i += 4) { a = max3_abs(a, v[i], v[i + 1]); b = max3_abs(b, v[i + 2], v[i + 3]); }
+  return fmaxf(a, b);
+}
+
 // ---- packed fp32 helpers (sm_100 has two-wide fp32 add / mul) ----------------------------------
 __device__ __forceinline__ void mul2(float a, float b, float s, float& d0, float& d1) {
   asm("{.reg .b64 p, q, r; mov.b64 p, {%2, %3}; mov.b64 q, {%4, %4}; mul.rn.f32x2 r, p, q; mov.b64 {%0, %1}, r;}"

@@ -1,0 +1,363 @@
+// Quantizers whose output describes x^T (blocks along the ROWS of x), alone or together with the row-wise output
+// of the same tensor, maxima given (sm_100a).
+//
+// What they serve: the transposed operands W^T, dY^T, X^T of FP4Linear (nvfp4_train.py:36-55) and every tensor that
+// is wanted in both layouts at once.  One persistent kernel walks over tiles of 128 rows x 128 columns of x.  A tile
+// arrives as two TMA tensor copies (128 x 64 elements, 128-byte swizzle, out-of-range elements read as zero) in one
+// of two 32 KiB slots; the next tile's copies are in flight while this one is encoded.
+//   row-wise     a lane takes a 16-element block: a warp covers rows {2w, 2w+1} + 32 g of a 128 x 64 half, so its 32
+//                scale bytes are one sector of the tiled layout and its codes eight full sectors
+//   transposed   a lane takes the 16 rows of two adjacent columns (a warp reads one 128-byte row of the half per
+//                instruction, no bank conflicts); the Hadamard butterflies of the two columns ride in the two lanes
+//                of packed fp32 instructions.  Codes and scales are collected in shared memory and leave as 64
+//                contiguous bytes per output row (two full sectors) and 1024 contiguous scale bytes.
+// A tensor of fewer tiles than the chip holds CTAs is cut finer: one CTA takes a tile's row-wise output, another its
+// transposed one (512 x 768, both stochastic: 6.0 -> 4.7 us; the whole tile per CTA wins once the grid is full).
+// What bounds it: the arithmetic pipes (about 200 instructions per block with Philox and the butterfly, half of them
+// on the half-rate ALU pipe), not memory.
+// Measured, maxima given, HBM-cold, us (before = one 64 x 64 tile per 256-thread CTA, and for the transposed output alone
+// two columns x 64 rows per thread straight from global memory):
+//   4096 x 28672   transposed nearest 68.2 -> 49.8, RHT 74.6 -> 61.1, RHT + stochastic 87.9 -> 85.7; both layouts
+//                  nearest 169.6 -> 98.4, stochastic 192.5 -> 143.9; a weight in both layouts 123.7 -> 83.6
+//   16384 x 768    transposed RHT + stochastic 17.2 -> 14.1, both layouts stochastic 24.4 -> 21.3
+//   512 x 768      transposed RHT + stochastic 6.6 -> 4.3, both layouts stochastic 4.0 -> 4.7, a weight 3.1 -> 3.8
+// Rows and columns outside the matrix get zero scale bytes, so the padding of the scale buffers needs no clearing.
+#include <mutex>
+
+#include "quantize_common.cuh"
+#include "gemm_common.cuh"      // encode_fn(): the driver's tensor-map encoder, looked up once
+
+namespace nvfp4 {
+namespace dual {
+
+using fused::PhiloxKeys;
+
+constexpr int kTile = 128;                        // rows and columns of x per tile
+constexpr int kThreads = 512;
+constexpr int kHalfBytes = kTile * 128;           // 128 rows x 64 columns
+constexpr int kSlotBytes = 2 * kHalfBytes;
+constexpr int kSlots = 2;
+constexpr int kOutPitch = 72;                     // 64 bytes of codes per output row, padded: 4 wavefronts per store
+constexpr int kOutBytes = kTile * kOutPitch + 1024;   // codes and scales of one tile's transposed output
+constexpr int kMiscOff = kSlots * kSlotBytes + 2 * kOutBytes;
+constexpr int kSmemBytes = kMiscOff + 1280 /* tables, signs, barriers */ + 1024 /* alignment slack */;
+
+struct Params {
+  int64_t rows, cols;
+  uint32_t ntc, nunits;          // column tiles per row of tiles; units of work in all
+  uint32_t split;                // 0: a unit is a tile; 1: units 2t and 2t + 1 are tile t's transposed and row-wise output
+  const float* signs16;
+  const float* amax_r;
+  const float* amax_c;
+  PhiloxKeys keys_r, keys_c;
+  uint64_t offset;
+  uint64_t pitch_r, base_r, pitch_c, base_c;      // Philox counter of a block = out_row * pitch + base + k_block
+  uint8_t* q_r;
+  uint8_t* sf_r;
+  float* pts_r;
+  uint8_t* q_c;
+  uint8_t* sf_c;
+  float* pts_c;
+};
+
+__device__ __forceinline__ void tma_half_load(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+
+__device__ __forceinline__ fused::Scale global_scale(float amax) {
+  fused::Scale s;
+  s.pts = __fdiv_rn(fmaxf(amax, kAmaxFloor), kGlobalDiv);
+  s.inv_pts = __fdiv_rn(1.0f, s.pts);
+  s.c = __fdiv_rn(1.0f, kF4Max * s.pts);
+  return s;
+}
+
+// v[16] -> codes and scale byte, the arithmetic of every quantizer here (quantize_common.cuh).
+// POSZERO: an exact zero that left the butterfly as -0 becomes +0
+template <bool SR, bool POSZERO>
+__device__ __forceinline__ void encode(const float (&v)[16], float amax_b, const fused::Scale& sc, const float* recip_tab,
+                                       uint64_t counter, const PhiloxKeys& keys, uint64_t offset, uint32_t& lo,
+                                       uint32_t& hi, uint32_t& sf) {
+  sf = fused::block_scale_byte(amax_b, sc);
+  const float recip = recip_tab[sf];
+  float d[16];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (POSZERO) fused::mul2_poszero(v[2 * j], v[2 * j + 1], recip, d[2 * j], d[2 * j + 1]);
+    else fused::mul2(v[2 * j], v[2 * j + 1], recip, d[2 * j], d[2 * j + 1]);
+  }
+  if (SR) {
+    const Philox4 r = fused::philox_rounds((uint32_t)counter, (uint32_t)(counter >> 32), (uint32_t)offset,
+                                           (uint32_t)(offset >> 32), keys);
+    lo = e2m1x4_rs(d[0], d[1], d[2], d[3], r.x) | (e2m1x4_rs(d[4], d[5], d[6], d[7], r.y) << 16);
+    hi = e2m1x4_rs(d[8], d[9], d[10], d[11], r.z) | (e2m1x4_rs(d[12], d[13], d[14], d[15], r.w) << 16);
+  } else {
+    lo = fused::e2m1x8_rn(d);
+    hi = fused::e2m1x8_rn(d + 8);
+  }
+}
+
+// ROWS: 0 no row-wise output, 1 round to nearest, 2 stochastic.  SR_C, RHT: rounding and random-sign Hadamard (along
+// the rows of x) of the transposed output.
+template <int ROWS, bool SR_C, bool RHT>
+__global__ void __launch_bounds__(kThreads, 2)
+quant_dual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = fused::smem_u32(smem_raw);
+  uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);          // the swizzle wants 1024-byte alignment
+  float* recip_r = reinterpret_cast<float*>(smem + kMiscOff);            // 128 floats each
+  float* recip_c = recip_r + 128;
+  uint32_t* sgn = reinterpret_cast<uint32_t*>(recip_c + 128);            // 16 sign-flip masks
+  const uint32_t bars = fused::smem_u32(sgn + 16);
+  volatile int* gave_up = reinterpret_cast<volatile int*>(sgn + 16 + 2 * kSlots);
+
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t my_tiles = blockIdx.x < p.nunits ? (p.nunits - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
+  auto locate = [&](uint32_t i, int64_t& r0, int64_t& c0) {
+    const uint32_t tile = (blockIdx.x + i * gridDim.x) >> p.split, rt = tile / p.ntc;
+    r0 = (int64_t)rt * kTile;
+    c0 = (int64_t)(tile - rt * p.ntc) * kTile;
+  };
+  auto fetch = [&](uint32_t i) {                  // one thread: both halves of this CTA's tile i into slot i % kSlots
+    int64_t r0, c0;
+    locate(i, r0, c0);
+    const uint32_t s = i % kSlots, bar = bars + 8u * s, dst = fused::smem_u32(smem) + s * kSlotBytes;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)kSlotBytes) : "memory");
+    tma_half_load(dst, &map_x, (int)c0, (int)r0, bar);
+    tma_half_load(dst + kHalfBytes, &map_x, (int)(c0 + 64), (int)r0, bar);
+  };
+  if (tid == 0) {
+    for (int s = 0; s < kSlots; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8u * s));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    *gave_up = 0;
+    for (uint32_t i = 0; i < (uint32_t)kSlots && i < my_tiles; ++i) fetch(i);
+  }
+  // scales and tables while the first tiles arrive
+  const fused::Scale sc_c = global_scale(__ldg(p.amax_c));
+  fused::Scale sc_r = sc_c;
+  if (ROWS) sc_r = global_scale(__ldg(p.amax_r));
+  // The transform is butterfly / 4.  The quarter is folded into the reciprocals (an exact scaling) unless that could
+  // make one a denormal: then (maxima above 1e38) the values take it.
+  const bool fold = !RHT || sc_c.inv_pts >= 4.0f * kE4M3Max * 1.17549435e-38f;
+  const float rht_scale = RHT && fold ? 0.25f : 1.0f;
+  if (tid < 128) recip_c[tid] = __fdiv_rn(sc_c.inv_pts, e4m3_to_f32(tid)) * rht_scale;
+  else if (ROWS && tid < 256) recip_r[tid - 128] = __fdiv_rn(sc_r.inv_pts, e4m3_to_f32(tid - 128));
+  else if (RHT && tid >= 256 && tid < 272) sgn[tid - 256] = __ldg(p.signs16 + (tid - 256)) < 0.0f ? 0x80000000u : 0u;
+  if (blockIdx.x == 0 && tid == 0) {
+    if (p.pts_c != nullptr) *p.pts_c = sc_c.pts;
+    if (ROWS && p.pts_r != nullptr) *p.pts_r = sc_r.pts;
+  }
+  __syncthreads();
+
+  const int64_t blk_r = p.cols >> 4, blk_c = p.rows >> 4;               // blocks per output row of the two layouts
+  const int64_t ct_r = (blk_r + 3) >> 2, ct_c = (blk_c + 3) >> 2;       // scale tiles per 128 output rows
+  for (uint32_t i = 0; i < my_tiles; ++i) {
+    int64_t r0, c0;
+    locate(i, r0, c0);
+    const uint32_t slot_off = (i % kSlots) * kSlotBytes, bar = bars + 8u * (i % kSlots), parity = (i / kSlots) & 1u;
+    if (!fused::mbar_try_wait(bar, parity)) {
+      const unsigned long long t0 = fused::global_ns();
+      while (!fused::mbar_try_wait(bar, parity)) {
+        if (fused::global_ns() - t0 > fused::kWaitLimitNs) { *gave_up = 1; break; }
+      }
+    }
+    const uint8_t* slot = smem + slot_off;
+    uint8_t* out = smem + kSlots * kSlotBytes + (i & 1u) * kOutBytes;
+    uint8_t* out_sf = out + kTile * kOutPitch;
+
+    const uint32_t part = (blockIdx.x + i * gridDim.x) & p.split;
+    const bool do_cols = ROWS == 0 || part == 0, do_rows = p.split == 0 || part != 0;
+    // ---- transposed: this warp's half and 16-row block, two columns per lane
+    if (do_cols) {
+      const uint32_t half = warp & 1u, rb = warp >> 1;
+      const uint32_t addr = fused::smem_u32(slot) + half * kHalfBytes + rb * 2048u + (lane & 3u) * 4u;
+      float v0[16], v1[16];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint4 m4 = make_uint4(0u, 0u, 0u, 0u);
+        if (RHT) m4 = reinterpret_cast<const uint4*>(sgn)[q];
+        const uint32_t m[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int k = 4 * q + e;
+          uint32_t w;
+          asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"((addr + (((lane >> 2) ^ (k & 7)) << 4)) + 128 * k));
+          v0[k] = __uint_as_float((w << 16) + m[e]);                     // adding the top bit flips the sign: one
+          v1[k] = __uint_as_float((w & 0xffff0000u) ^ m[e]);             // instruction each with the unpacking
+        }
+      }
+      if (RHT) {
+#pragma unroll
+        for (int s = 1; s < 16; s <<= 1) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k)
+            if ((k & s) == 0) fused::addsub2(v0[k], v1[k], v0[k | s], v1[k | s]);
+        }
+        if (!fold) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) fused::mul2(v0[k], v1[k], 0.25f, v0[k], v1[k]);
+        }
+      }
+      const int64_t kb = (r0 >> 4) + rb;
+      const uint32_t c = half * 64u + 2u * lane;                         // column inside the tile
+      const uint64_t ctr = (uint64_t)(c0 + c) * p.pitch_c + p.base_c + (uint64_t)kb;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float(&v)[16] = h ? v1 : v0;
+        uint32_t lo, hi, sf;
+        encode<SR_C, RHT>(v, fused::max_abs16(v) * rht_scale, sc_c, recip_c, ctr + (h ? p.pitch_c : 0ull), p.keys_c,
+                          p.offset, lo, hi, sf);
+        *reinterpret_cast<uint2*>(out + (c + h) * kOutPitch + rb * 8u) = make_uint2(lo, hi);
+        const bool inside = c0 + c + h < p.cols && kb < blk_c;
+        out_sf[(rb >> 2) * 512u + ((c + h) & 31u) * 16u + ((c + h) >> 5) * 4u + (rb & 3u)] = inside ? (uint8_t)sf : (uint8_t)0;
+      }
+    }
+    // ---- row-wise: blocks (row_t, kb) of the two halves
+    if (ROWS && do_rows) {
+      const uint32_t kb4 = lane & 3u, hrow = (lane >> 2) & 1u, grp = lane >> 3;
+      const uint32_t row_t = 2u * warp + hrow + 32u * grp;
+      const uint32_t off0 = row_t * 128u + (((2u * kb4) ^ (row_t & 7u)) << 4);
+      const uint32_t off1 = row_t * 128u + (((2u * kb4 + 1u) ^ (row_t & 7u)) << 4);
+      const int64_t r = r0 + row_t;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        if (c0 + 64 * half >= p.cols) break;                             // no such scale tile (uniform)
+        const int64_t kb = (c0 >> 4) + 4 * half + kb4;
+        const uint4 a = *reinterpret_cast<const uint4*>(slot + half * kHalfBytes + off0);
+        const uint4 b = *reinterpret_cast<const uint4*>(slot + half * kHalfBytes + off1);
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { v[2 * j] = bf16_lo(w[j]); v[2 * j + 1] = bf16_hi(w[j]); }
+        uint32_t lo, hi, sf;
+        encode<ROWS == 2, false>(v, fused::amax_packed8(w), sc_r, recip_r,
+                                 (uint64_t)r * p.pitch_r + p.base_r + (uint64_t)kb, p.keys_r, p.offset, lo, hi, sf);
+        const bool inside = r < p.rows && kb < blk_r;
+        if (inside) *reinterpret_cast<uint2*>(p.q_r + r * (p.cols >> 1) + kb * 8) = make_uint2(lo, hi);
+        p.sf_r[((r0 >> 7) * ct_r + (c0 >> 6) + half) * 512 + (2u * warp + hrow) * 16u + grp * 4u + kb4] =
+            inside ? (uint8_t)sf : (uint8_t)0;
+      }
+    }
+    __syncthreads();                                                     // the slot is read, the output collected
+    if (*gave_up != 0) return;
+    if (tid == 0 && i + kSlots < my_tiles) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // generic reads before the async write
+      fetch(i + kSlots);
+    }
+    // ---- transposed output: thread t writes 16 of the 64 bytes of output row t / 4; 64 threads write the scales
+    if (do_cols) {
+      const uint32_t row = tid >> 2, b16 = (tid & 3u) * 16u;
+      const int64_t oc = c0 + row, k_byte = (r0 >> 1) + b16, out_ld = p.rows >> 1;
+      if (oc < p.cols && k_byte < out_ld) {
+        const uint2 a = *reinterpret_cast<const uint2*>(out + row * kOutPitch + b16);
+        const uint2 b = *reinterpret_cast<const uint2*>(out + row * kOutPitch + b16 + 8);
+        uint8_t* dst = p.q_c + oc * out_ld + k_byte;
+        if ((out_ld & 15) == 0) {
+          *reinterpret_cast<uint4*>(dst) = make_uint4(a.x, a.y, b.x, b.y);
+        } else {                                                         // rows of 8-byte multiples
+          *reinterpret_cast<uint2*>(dst) = a;
+          if (k_byte + 8 < out_ld) *reinterpret_cast<uint2*>(dst + 8) = b;
+        }
+      }
+      if (tid < 64 && (r0 >> 6) + (tid >> 5) < ct_c)
+        *reinterpret_cast<uint4*>(p.sf_c + ((c0 >> 7) * ct_c + (r0 >> 6)) * 512 + tid * 16u) =
+            *reinterpret_cast<const uint4*>(out_sf + tid * 16u);
+    }
+  }
+}
+
+namespace {
+std::mutex g_mutex;
+int g_sms[64];
+
+const void* kernel_fn(int rows_mode, bool sr_c, bool rht) {
+#define NVFP4_DUAL_FN(R_) \
+  (sr_c ? (rht ? (const void*)quant_dual_kernel<R_, true, true> : (const void*)quant_dual_kernel<R_, true, false>) \
+        : (rht ? (const void*)quant_dual_kernel<R_, false, true> : (const void*)quant_dual_kernel<R_, false, false>))
+  return rows_mode == 0 ? NVFP4_DUAL_FN(0) : (rows_mode == 1 ? NVFP4_DUAL_FN(1) : NVFP4_DUAL_FN(2));
+#undef NVFP4_DUAL_FN
+}
+
+int sm_count(int& out) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return NVFP4_E_LAUNCH;
+  std::lock_guard<std::mutex> lock(g_mutex);
+  if (g_sms[dev] == 0) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return NVFP4_E_LAUNCH;
+    for (int v = 0; v < 12; ++v)
+      if (cudaFuncSetAttribute(kernel_fn(v >> 2, (v & 2) != 0, (v & 1) != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               kSmemBytes) != cudaSuccess) {
+        cudaGetLastError();
+        return NVFP4_E_LAUNCH;
+      }
+    g_sms[dev] = sms;
+  }
+  out = g_sms[dev];
+  return NVFP4_OK;
+}
+}  // namespace
+
+static PhiloxKeys make_keys(uint64_t seed) {
+  PhiloxKeys keys;
+  for (int r = 0; r < 10; ++r) {
+    keys.k[r][0] = (uint32_t)seed + (uint32_t)r * 0x9E3779B9u;
+    keys.k[r][1] = (uint32_t)(seed >> 32) + (uint32_t)r * 0xBB67AE85u;
+  }
+  return keys;
+}
+
+// x [rows, cols] bf16, row pitch ld elements; rows_mode 0 / 1 / 2 = no row-wise output / nearest / stochastic; signs16
+// null = no Hadamard on the transposed output.  counters4 = pitch_r, base_r, pitch_c, base_c.  Arguments have been
+// validated by the caller (quantize.cu): 16-byte aligned pointers, ld % 8 == 0, rows % 16 == 0, and cols % 16 == 0 when
+// there is a row-wise output.
+int launch(const void* x, int64_t rows, int64_t cols, int64_t ld, int rows_mode, bool sr_c, const float* signs16,
+           const float* amax_r, const float* amax_c, uint64_t seed_r, uint64_t seed_c, uint64_t offset,
+           const uint64_t* counters4, uint8_t* q_r, uint8_t* sf_r, float* pts_r, uint8_t* q_c, uint8_t* sf_c, float* pts_c,
+           cudaStream_t stream) {
+  int sms = 0;
+  const int rc = sm_count(sms);
+  if (rc != NVFP4_OK) return rc;
+  gemm::EncodeTiledFn enc = gemm::encode_fn();
+  if (enc == nullptr) return NVFP4_E_DRIVER;
+  CUtensorMap map;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 2u};
+  cuuint32_t box[2] = {64u, (cuuint32_t)kTile};
+  cuuint32_t estr[2] = {1u, 1u};
+  if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
+          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return NVFP4_E_DRIVER;
+  Params p;
+  p.rows = rows;
+  p.cols = cols;
+  const int64_t ntc = (cols + kTile - 1) / kTile, ntiles = ntc * ((rows + kTile - 1) / kTile);
+  if (ntiles >= (1ll << 30)) return NVFP4_E_LIMIT;
+  p.ntc = (uint32_t)ntc;
+  // (three half units of work per SM at most are better balanced than two whole ones)
+  p.split = rows_mode != 0 && ntiles <= 2 * sms ? 1u : 0u;
+  p.nunits = (uint32_t)ntiles << p.split;
+  p.signs16 = signs16;
+  p.amax_r = amax_r;
+  p.amax_c = amax_c;
+  p.keys_r = make_keys(seed_r);
+  p.keys_c = make_keys(seed_c);
+  p.offset = offset;
+  p.pitch_r = counters4[0]; p.base_r = counters4[1]; p.pitch_c = counters4[2]; p.base_c = counters4[3];
+  p.q_r = q_r; p.sf_r = sf_r; p.pts_r = pts_r;
+  p.q_c = q_c; p.sf_c = sf_c; p.pts_c = pts_c;
+  const uint32_t grid = p.nunits < 2u * (uint32_t)sms ? p.nunits : 2u * (uint32_t)sms;      // two resident CTAs per SM
+  void* args[] = {&map, &p};
+  if (cudaLaunchKernel(kernel_fn(rows_mode, sr_c, signs16 != nullptr), dim3(grid), dim3(kThreads), args, kSmemBytes,
+                       stream) != cudaSuccess) {
+    cudaGetLastError();          // a refused launch must not show up as the next call's error
+    return NVFP4_E_LAUNCH;
+  }
+  return NVFP4_OK;
+}
+
+}  // namespace dual
+}  // namespace nvfp4

@@ -112,9 +112,7 @@ quant_fused_kernel(const uint16_t* __restrict__ x, uint32_t rows, uint32_t blk_p
     if (RHT) {
       float v[16];
       expand<true>(w, sm, v);
-      float a = 0.0f;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) a = fmaxf(a, fabsf(v[j]));
+      float a = max_abs16(v);
       return a * 0.25f;
     }
     const float a = amax_packed8(w);
@@ -224,9 +222,7 @@ quant_fused_kernel(const uint16_t* __restrict__ x, uint32_t rows, uint32_t blk_p
     float amax_b;
     if (RHT) {
       expand<true>(w, sm, v);
-      amax_b = 0.0f;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) amax_b = fmaxf(amax_b, fabsf(v[j]));
+      amax_b = max_abs16(v);
       amax_b *= 0.25f;                                   // H = butterfly / 4, an exact scaling
     } else {
       expand<false>(w, sm, v);

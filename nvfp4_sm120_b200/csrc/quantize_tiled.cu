@@ -239,9 +239,7 @@ quant_tiled_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
         if (RHT) {
           float v[16];
           expand<true>(w[e], sm, v);
-          a = 0.0f;
-#pragma unroll
-          for (int j = 0; j < 16; ++j) a = fmaxf(a, fabsf(v[j]));
+          a = max_abs16(v);
           a *= 0.25f;
         } else {
           a = amax_packed8(w[e]);
@@ -329,9 +327,7 @@ quant_tiled_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
       float amax_b;
       if (RHT) {
         expand<true>(w[e], sm, v);
-        amax_b = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) amax_b = fmaxf(amax_b, fabsf(v[j]));
+        amax_b = max_abs16(v);
         amax_b *= 0.25f;                                   // H = butterfly / 4, an exact scaling
       } else {
         expand<false>(w[e], sm, v);

@@ -72,3 +72,21 @@ def test_dual_with_shard_counters(Q):
                                       True, True, 21, 22, counters=ctr)
         assert torch.equal(d_r.qdata, a_r.qdata[:, rank * nl // 2:(rank + 1) * nl // 2])
         assert torch.equal(d_c.qdata, a_c.qdata[rank * nl:(rank + 1) * nl])
+
+
+@pytest.mark.parametrize("shape", [(16, 2), (128, 128), (144, 130), (272, 24), (4112, 264)])
+@pytest.mark.parametrize("sr,rht", [(False, False), (False, True), (True, True)])
+def test_transposed_edges_against_the_oracle(Q, shape, sr, rht):
+    """Tiles of 128 x 128 that end inside the matrix, and a row pitch wider than the matrix."""
+    rows, cols = shape
+    x = O.synthetic_tensor(rows, cols, 74)
+    signs = O.signs_from_seed(2)
+    wide = torch.zeros(rows, (cols + 15) // 8 * 8, dtype=torch.bfloat16, device="cuda")
+    wide[:, :cols] = x.cuda()
+    rb = O.philox_block_bits(rows * cols // 16, 9, 0)
+    want = O.quant_nvfp4(x.t().contiguous(), stochastic=sr, rht=rht, signs=signs, rbits=rb if sr else None,
+                         rht_impl="butterfly")
+    amax = None if rht else wide.float().abs().max().reshape(1)      # (the plain maximum kernel wants cols % 8 == 0)
+    got = Q.quant_nvfp4(wide[:, :cols], sr, rht, signs=signs.cuda(), seed=9, transpose=True, amax=amax)
+    assert torch.equal(got.qdata.cpu(), want.qdata)
+    assert torch.equal(got.scale.view(torch.uint8).cpu(), want.scale.view(torch.uint8))
