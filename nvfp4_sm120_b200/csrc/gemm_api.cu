@@ -2,11 +2,11 @@
 #include "gemm_common.cuh"
 
 namespace nvfp4 { namespace gemm3 {
-int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_d, const gemm::Params& p,
+int launch_pair(int tile_n, const CUtensorMap& map_d, const uint8_t* a_q, const uint8_t* b_q, const gemm::Params& p,
                 cudaStream_t stream);
 }}
 namespace nvfp4 { namespace gemm {
-int launch_1cta(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_d, const Params& p,
+int launch_1cta(int tile_n, const CUtensorMap& map_d, const uint8_t* a_q, const uint8_t* b_q, const Params& p,
                 cudaStream_t stream);
 }}
 
@@ -28,9 +28,6 @@ extern "C" int nvfp4_gemm_set_mode(int mode) {
   return NVFP4_OK;
 }
 
-// Automatic choice: the persistent pair kernel (mode 2), which measured fastest on every shape with
-// more than one row tile; the one-CTA kernel (mode 1) when M <= 128 (a pair would compute 128 rows of
-// padding) and for the split-K case below.  Modes 1 and 2 force a kernel, for tuning and tests.
 namespace nvfp4 { namespace gemm {
 __global__ void pts_from_amax_kernel(const float* __restrict__ amax, float* __restrict__ pts) {
   *pts = __fdiv_rn(fmaxf(*amax, kAmaxFloor), kGlobalDiv);
@@ -40,6 +37,53 @@ int launch_pts_from_amax(const float* amax, float* pts, cudaStream_t stream) {
   return cudaGetLastError() == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
 }
 }}
+
+// Kernel, tile width and CTAs per tile.
+struct Choice { bool pair; int tile_n, splits; };
+
+// The rule: the candidate with the smallest estimate of its time in us,
+//   fixed part + waves * K slices per CTA * time per slice + drain of the waves before the last (+ sum over the cluster),
+// with constants measured on a B200 (CUDA graph of 24 launches, operands in L2) over 1 .. 16384 x 300 .. 14336 x 512 ..
+// 16384: launch, pipeline fill and epilogue 3.8 us for a 128 x 64 tile, 5.75 us for a 256 x 256 pair; a slice is bound by
+// the fill of shared memory from L2 (about 64 bytes per SM and clock) in the one-CTA kernel, by the shared-memory data
+// stage in the pair kernel.  The estimate orders the candidates right where they differ by more than about 5 %.  Where
+// the lines fall (us, best candidate against the 256 x 256 pair tiles): 512 x 768 x 768 4.9 / 6.8 (128 x 64), 5328 x 768 x
+// 768 6.7 / 7.2 (128 x 256), 2048 x 768 x 3072 8.6 / 9.8 (pair 256 x 128), 1000 x 2584 x 7136 17.0 / 18.6 (pair 256 x 192),
+// 256 x 1024 x 8192 8.9 / 14.9 (128 x 64, four CTAs per tile), 64 x 4096 x 14336 12.6 / 22.9 (128 x 128, four),
+// 768 x 768 x 16384 15.3 / 24.7 (128 x 64, two), 8 x 14336 x 4096 11.9 / 12.6 (128 x 256, two).
+static Choice choose(int64_t M, int64_t N, int64_t K, int forced, bool may_split) {
+  struct Kind { bool pair; int tile_n; float fixed, slice, drain, sum; };
+  static const Kind kinds[] = {{true, 256, 5.75f, 0.315f, 1.3f, 0.0f}, {true, 192, 5.35f, 0.31f, 0.85f, 0.0f},
+                               {true, 128, 4.75f, 0.29f, 0.6f, 0.0f},  {false, 256, 5.35f, 0.39f, 4.3f, 2.6f},
+                               {false, 128, 4.25f, 0.345f, 3.8f, 1.6f}, {false, 64, 3.8f, 0.32f, 2.4f, 1.2f}};
+  // CTAs that the device holds at once as clusters of 1, 2, 4, 8 (clusters of 8: 16 of them did not fit)
+  static const int caps[] = {148, 148, 128, 112};
+  const int64_t slices = (K + 255) / 256;
+  Choice best{true, 256, 1};
+  float best_us = 3.0e38f;
+#ifdef NVFP4_TUNE
+  if (const char* e = getenv("NVFP4_TUNE")) {
+    int v = atoi(e), sp = 1;
+    if (const char* c = strchr(e, ',')) sp = atoi(c + 1);
+    if ((slices + sp - 1) / sp * (sp - 1) >= slices) sp = 1;
+    return Choice{v < 0, v < 0 ? -v : v, sp};
+  }
+#endif
+  for (const Kind& k : kinds) {
+    if (forced != 0 && k.pair != (forced == 2)) continue;
+    const int64_t rows = k.pair ? 256 : 128, tiles = ((M + rows - 1) / rows) * ((N + k.tile_n - 1) / k.tile_n);
+    for (int log_s = 0; log_s < (k.pair || !may_split ? 1 : 4); ++log_s) {
+      const int s = 1 << log_s;
+      const int64_t per = (slices + s - 1) / s, cap = k.pair ? 74 : caps[log_s];
+      if (s > 1 && (tiles * s > cap || per * (s - 1) >= slices)) break;      // one wave, and work for every CTA
+      const int64_t waves = (tiles * s + cap - 1) / cap;
+      float us = k.fixed + (float)waves * (float)per * k.slice + (float)(waves - 1) * k.drain;
+      if (s > 1) us += 0.3f + 0.15f * (float)s + k.sum * (float)(M < 128 ? M : 128) / 128.0f;
+      if (us < best_us) { best_us = us; best = Choice{k.pair, k.tile_n, s}; }
+    }
+  }
+  return best;
+}
 
 static int gemm_any(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pts, const uint8_t* b_q,
                     const uint8_t* b_sf, const float* b_pts, void* d, int out_dtype, int64_t M, int64_t N,
@@ -54,47 +98,24 @@ static int gemm_any(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pts,
   if (out_dtype != NVFP4_OUT_BF16 && out_dtype != NVFP4_OUT_F32) return NVFP4_E_MODE;
   auto mis = [](const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) != 0; };
   if (mis(a_q, 16) || mis(b_q, 16) || mis(a_sf, 16) || mis(b_sf, 16) || mis(d, 16)) return NVFP4_E_ALIGN;
-  // split K (one-CTA kernel only, see below) when a small fp32 output would leave most SMs idle
-  const int64_t tiles_1cta = ((N + 255) / 256) * ((M + 127) / 128), slices = (K + 255) / 256;
-  // (partial sums have no maximum of their own: no split when the caller wants max|D|)
-  const bool want_split = out_dtype == NVFP4_OUT_F32 && tiles_1cta <= 74 && slices >= 16 && d_amax_out == nullptr;
   if (d_amax_out != nullptr) {
     if (fp4_out) return NVFP4_E_MODE;
     if (cudaMemsetAsync(d_amax_out, 0, sizeof(float), stream) != cudaSuccess) return NVFP4_E_LAUNCH;
   }
   const int forced = g_gemm_mode.load(std::memory_order_relaxed);
-  const int mode = forced != 0 ? forced : ((M > 128 && !want_split) ? 2 : 1);
-  const bool pair = mode == 2;
-  CUtensorMap map_a, map_b;
-  if (!make_operand_map(&map_a, a_q, M, K, 128) || !make_operand_map(&map_b, b_q, N, K, pair ? 128 : 256))
-    return NVFP4_E_DRIVER;
-  Params p{a_sf, b_sf, a_pts, b_pts, d, M, N, K, ldd, out_dtype == NVFP4_OUT_F32 ? 1 : 0, status, 1, 0,
+  // (a shared tile is stored by the cluster's sum: no maximum, no quantized output there)
+  const Choice pick = choose(M, N, K, forced, !fp4_out && d_amax_out == nullptr);
+  Params p{a_sf, b_sf, a_pts, b_pts, d, M, N, K, ldd, out_dtype == NVFP4_OUT_F32 ? 1 : 0, status, pick.splits, 0,
            g_gemm_wait_ns.load(std::memory_order_relaxed), g_gemm_drop_arrival.load(std::memory_order_relaxed),
            d_sf, d_amax, fp4_out ? 1 : 0, d_amax_out};
-  // Split K when a small fp32 output (the weight gradient: few tiles, K = tokens) would leave most SMs
-  // idle: the CTAs of a tile add their partial sums into the zeroed output.  Summation order then
-  // varies from run to run in the last bits, so it is used only where it pays: fewer tiles than half
-  // the SMs and at least 16 K slices (8 or more per CTA).
-  if (!pair && want_split) {
-    {
-      int64_t s = 148 / tiles_1cta;
-      if (s > slices / 8) s = slices / 8;              // at least 8 slices per CTA
-      if (s > 1) {
-        p.splits = (int)s;
-        cudaError_t e = (ldd == N) ? cudaMemsetAsync(d, 0, (size_t)M * N * 4, stream)
-                                   : cudaMemset2DAsync(d, (size_t)ldd * 4, 0, (size_t)N * 4, (size_t)M, stream);
-        if (e != cudaSuccess) return NVFP4_E_LAUNCH;
-      }
-    }
-  }
-  // The epilogue stores through TMA when the row pitch allows a tensor map (a multiple of 16 bytes)
-  // and the output is written, not accumulated into.
-  CUtensorMap map_d = map_a;                                   // placeholder when unused
+  // The epilogue stores through TMA when the row pitch allows a tensor map (a multiple of 16 bytes).
+  CUtensorMap map_d{};                                         // unused otherwise
   if (p.splits == 1 && !fp4_out && (ldd * (p.out_f32 ? 4 : 2)) % 16 == 0) {
     if (!make_output_map(&map_d, d, M, N, ldd, p.out_f32 != 0)) return NVFP4_E_DRIVER;
     p.tma_store = 1;
   }
-  return pair ? nvfp4::gemm3::launch_pair(map_a, map_b, map_d, p, stream) : launch_1cta(map_a, map_b, map_d, p, stream);
+  return pick.pair ? nvfp4::gemm3::launch_pair(pick.tile_n, map_d, a_q, b_q, p, stream)
+              : launch_1cta(pick.tile_n, map_d, a_q, b_q, p, stream);
 }
 
 extern "C" int nvfp4_gemm(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pts, const uint8_t* b_q,

@@ -13,7 +13,7 @@ constexpr int kTmemCols = 512;
 constexpr int kGroupM = 32;                 // row tiles per rasterization group (32 measured 1-3 % above 16, 8 below)
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;   // a wait that lasts 2 s gives up (the default)
 
-enum : int { kErrProducerWait = 1, kErrMmaWait = 2, kErrEpilogueWait = 3, kErrScaleWait = 4 };
+enum : int { kErrProducerWait = 1, kErrMmaWait = 2, kErrEpilogueWait = 3 };
 
 // ---- PTX wrappers -------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -153,12 +153,11 @@ struct Params {
   int64_t M, N, K, ldd;
   int out_f32;
   int32_t* status;
-  int splits;        // > 1: K is split over `splits` CTAs per tile, which add their partial sums into
-                     // a zeroed fp32 output with atomics (one-CTA kernel only)
+  int splits;        // > 1: the K slices of a tile are shared by a cluster of `splits` CTAs (one-CTA kernel only)
   int tma_store;     // the output goes through shared memory and TMA stores (needs a 16-byte row pitch)
   unsigned long long wait_limit_ns;   // every bounded wait gives up after this long (0 = kWaitLimitNs)
-  int drop_first_scale_arrival;       // test hook: the scale warps never announce K slice 0, so the MMA
-                                      // issuer's first wait runs out and the kernel takes its abort path
+  int drop_first_scale_arrival;       // test hook: the MMA issuer waits for an arrival that never comes, so that wait
+                                      // runs out and the kernel takes its abort path
   // NVFP4 output (out_fp4 != 0): d is the packed E2M1 buffer [M, N/2]; the bf16 rounding of every
   // output row is quantized in blocks of 16 along N with the per-tensor maximum *d_amax given
   uint8_t* d_sf;                      // swizzled E4M3 scales of the [M, N] operand
@@ -241,21 +240,6 @@ __device__ __forceinline__ void store_row_chunk(const Params& p, int64_t row, in
     // a row of N / 2 bytes starts on an 8-byte boundary (N % 16 == 0), not always on a 16-byte one
     *reinterpret_cast<uint2*>(q) = make_uint2(w[0], w[1]);
     if (full) *reinterpret_cast<uint2*>(q + 8) = make_uint2(w[2], w[3]);
-    return;
-  }
-  if (p.splits > 1) {                                   // split-K partial sum (fp32 output only)
-    float* out = static_cast<float*>(p.d) + row * p.ldd + col;
-    if (full && ((p.ldd & 3) == 0)) {                   // four floats per reduction instruction
-#pragma unroll
-      for (int j = 0; j < 32; j += 4)
-        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
-                     ::"l"(out + j), "f"(__uint_as_float(r[j]) * alpha), "f"(__uint_as_float(r[j + 1]) * alpha),
-                       "f"(__uint_as_float(r[j + 2]) * alpha), "f"(__uint_as_float(r[j + 3]) * alpha) : "memory");
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (col + j < p.N) atomicAdd(out + j, __uint_as_float(r[j]) * alpha);
-    }
     return;
   }
   if (p.out_f32) {

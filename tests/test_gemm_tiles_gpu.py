@@ -1,0 +1,43 @@
+"""Every kernel, tile width and cluster size that the GEMM's rule can choose, at sizes with ragged tiles, against a
+64-bit matmul of the dequantised operands.  Tolerance: fp32 accumulation of K products whose rounding errors are
+independent, about sqrt(K) * 2^-24 of the result's norm, K <= 14336: 7e-6; stated 1e-5."""
+import pytest
+import torch
+
+from oracle import nvfp4_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def Q():
+    import nvfp4_sm120_b200 as pkg
+    return pkg
+
+
+def _dequant(q):
+    rows, k = q.qdata.shape[0], q.qdata.shape[1] * 2
+    return O.dequant_parts(q.qdata, q.scale.view(torch.uint8), q.per_tensor_scale, rows, k).double().cuda()
+
+
+@pytest.mark.parametrize("mnk", [
+    (512, 768, 768), (129, 72, 256), (1, 8, 32),              # 128 x 64 tiles, odd column halves of a scale group
+    (300, 2088, 544), (1024, 4104, 992),                      # 128 x 128, 128 x 256
+    (2040, 776, 3104), (1000, 2584, 2080), (3000, 3000, 800),  # pair, 256 x 128 / 192 / 256, several tiles per pair
+    (300, 520, 8000), (33, 72, 4128), (8, 3000, 4096),        # shared tiles: clusters of 4, 8, 2
+    (64, 1096, 14336), (768, 768, 8192), (127, 2000, 8224)])
+def test_rule_choices_match_the_dequantised_product(Q, mnk):
+    m, n, k = mnk
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    qa = Q.quant_nvfp4(torch.randn(m, k, device="cuda", generator=g).bfloat16())
+    qb = Q.quant_nvfp4(torch.randn(n, k, device="cuda", generator=g).bfloat16()).t()
+    want = _dequant(qa) @ _dequant(qb).t()
+    f32 = Q.nvfp4_mm(qa, qb, torch.float32)
+    bf16 = Q.nvfp4_mm(qa, qb, torch.bfloat16)
+    assert Q.gemm_status() == 0
+    assert ((f32.double() - want).norm() / want.norm()).item() < 1e-5
+    assert torch.equal(bf16, f32.to(torch.bfloat16))          # one rounding of the same accumulators
+    assert torch.equal(f32, Q.nvfp4_mm(qa, qb, torch.float32))     # the same bits on every run
+    wide = torch.full((m, n + 8), 7.0, device="cuda")         # nothing is written outside the result
+    Q.nvfp4_mm(qa, qb, torch.float32, out=wide[:, :n])
+    assert torch.equal(wide[:, :n], f32) and bool((wide[:, n:] == 7.0).all())
