@@ -94,6 +94,27 @@ def lib():
     return _lib
 
 
+HOST_PATH = os.path.join(_PKG, "_host.so")
+_host = None
+
+
+def host():
+    """The native host side (csrc/host/host.cpp), bound to the library that lib() loads.  Raises if it has not
+    been built."""
+    global _host
+    if _host is None:
+        if not os.path.exists(HOST_PATH):
+            raise NVFP4Error(f"{HOST_PATH} is missing: build it with `python -m nvfp4_sm120_b200.build`")
+        import importlib.util
+        lib()
+        spec = importlib.util.spec_from_file_location("_host", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.init(LIB_PATH, check, cuda_device_of)
+        _host = module
+    return _host
+
+
 def exported_symbols():
     return list(_SIGS)
 

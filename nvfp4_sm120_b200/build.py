@@ -12,6 +12,7 @@ import sys
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 LIB = os.path.join(PKG, "libnvfp4_b200.so")
+HOST = os.path.join(PKG, "_host.so")               # native host side of the Python entry points (csrc/host)
 CLI = os.path.join(PKG, "nvfp4_gemm_cli")          # stand-alone C driver of the ABI (csrc/tools)
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared", "--threads", "4"]
@@ -23,13 +24,14 @@ def sources():
 
 def _deps():
     return sources() + glob.glob(os.path.join(PKG, "csrc", "*.cuh")) + \
-        glob.glob(os.path.join(ROOT, "include", "*.h")) + glob.glob(os.path.join(PKG, "csrc", "tools", "*.cu"))
+        glob.glob(os.path.join(ROOT, "include", "*.h")) + glob.glob(os.path.join(PKG, "csrc", "tools", "*.cu")) + \
+        glob.glob(os.path.join(PKG, "csrc", "host", "*.cpp"))
 
 
 def up_to_date():
-    if not os.path.exists(LIB) or not os.path.exists(CLI):
+    if not all(os.path.exists(p) for p in (LIB, CLI, HOST)):
         return False
-    t = os.path.getmtime(LIB)
+    t = min(os.path.getmtime(LIB), os.path.getmtime(HOST))
     return all(os.path.getmtime(p) <= t for p in _deps())
 
 
@@ -55,7 +57,27 @@ def build(force=False, verbose=False):
     res = subprocess.run(cli_cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("nvcc failed on the C driver:\n" + res.stdout + res.stderr)
+    build_host()
     return LIB
+
+
+def build_host():
+    """The pybind11 module beside the library: compiled by g++ against the installed torch (no GPU code in it)."""
+    import sysconfig
+    import torch
+    cxx = shutil.which("g++")
+    if cxx is None:
+        raise RuntimeError("g++ not found: cannot build _host.so")
+    t = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-I", os.path.join(ROOT, "include"),
+           "-isystem", os.path.join(t, "include"), "-isystem", os.path.join(t, "include", "torch", "csrc", "api", "include"),
+           "-isystem", os.path.join(cuda, "include"), "-isystem", sysconfig.get_paths()["include"],
+           os.path.join(PKG, "csrc", "host", "host.cpp"), "-o", HOST,
+           "-L", os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed on the host module:\n" + res.stdout + res.stderr)
 
 
 if __name__ == "__main__":

@@ -5,24 +5,17 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from .quant import quant_nvfp4, _stream
+from .quant import quant_nvfp4, _device_index, _stream
 from .tensor import NVFP4Tensor
-
-_STATUS = {}
 
 
 def _status_word(device):
-    if device not in _STATUS:
-        _STATUS[device] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _STATUS[device]
+    return _lib.host().status_word(_device_index(device))
 
 
 def gemm_status(device=None) -> int:
     """Device status word of the GEMM kernels on `device`: 0, or the code of the first bounded
     wait that gave up.  Reading it synchronises."""
-    device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    if device.index is None:
-        device = torch.device("cuda", torch.cuda.current_device())
     return int(_status_word(device).item())
 
 
@@ -48,19 +41,8 @@ def nvfp4_mm(a: NVFP4Tensor, b: NVFP4Tensor, out_dtype=None, out=None, amax_out=
         raise ValueError("out_dtype must be bfloat16 or float32")
     if amax_out is not None and (amax_out.dtype != torch.float32 or amax_out.numel() != 1):
         raise ValueError("amax_out must be a 1-element float32 tensor")
-    dev = _lib.cuda_device_of(a.qdata, a.scale, a.per_tensor_scale, b.qdata, b.scale, b.per_tensor_scale, out, amax_out)
-    d = out if out is not None else torch.empty((m, n), dtype=out_dtype, device=dev)
-    args = (a.qdata.data_ptr(), a.scale.data_ptr(), a.per_tensor_scale.data_ptr(),
-            b.qdata.data_ptr(), b.scale.data_ptr(), b.per_tensor_scale.data_ptr(),
-            d.data_ptr(), _lib.OUT_F32 if out_dtype == torch.float32 else _lib.OUT_BF16,
-            m, n, k2 * 2, d.stride(0))
-    with torch.cuda.device(dev):                   # the C side launches on the current device
-        if amax_out is None:
-            code = _lib.lib().nvfp4_gemm(*args, _status_word(dev).data_ptr(), _stream(dev))
-        else:
-            code = _lib.lib().nvfp4_gemm_amax(*args, amax_out.data_ptr(), _status_word(dev).data_ptr(), _stream(dev))
-    _lib.check(code, "nvfp4_gemm")
-    return d
+    return _lib.host().mm(a.qdata, a.scale, a.per_tensor_scale, b.qdata, b.scale, b.per_tensor_scale,
+                          out_dtype == torch.float32, out, amax_out)
 
 
 def nvfp4_mm_fp4out(a: NVFP4Tensor, b: NVFP4Tensor, out_amax: torch.Tensor) -> NVFP4Tensor:

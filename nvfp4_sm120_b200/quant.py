@@ -7,13 +7,12 @@ import math
 import torch
 
 from . import _lib
-from .tensor import BLK, NVFP4Tensor, swizzled_scale_dims
+from .tensor import BLK, NVFP4Tensor
 
 F4_MAX, F8E4M3_MAX, E4M3_EPS = 6.0, 448.0, 0.015625
 
 _SEED = [0]          # auto-advancing seed of stochastic calls, like nvfp4_cuda.py:154,160-162
 _H_OK = {}           # H tensors already checked to be the Sylvester matrix / 4
-_ONES = {}
 
 
 def hadamard16(device="cuda"):
@@ -38,36 +37,29 @@ def _check_h(H):
 
 
 def _signs(signs, device):
-    if signs is None:
-        if device not in _ONES:
-            _ONES[device] = torch.ones(BLK, device=device, dtype=torch.float32)
-        return _ONES[device]
+    """A sign vector as the kernels read it (the activation and norm wrappers)."""
     s = signs.to(device=device, dtype=torch.float32).contiguous()
     if s.numel() != BLK:
         raise ValueError("signs must have 16 entries")
     return s
 
 
-_WS = {}
+def _device_index(device):
+    index = None if device is None else torch.device(device).index
+    return torch.cuda.current_device() if index is None else index
 
 
 def _workspace(device):
     """64-byte scratch of the single-launch quantizer, zeroed once, one per (device, stream): every
     launch leaves it ready for the next, and launches on one stream never overlap."""
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
-    if key not in _WS:
-        _WS[key] = torch.zeros(16, dtype=torch.int32, device=device)
-    return _WS[key]
+    return _lib.host().workspace(_device_index(device))
 
 
 def fused_error(device=None) -> int:
     """Sticky error word of the single-launch quantizer's workspace on the current stream
     (0 = none).  Reading it synchronises."""
-    device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    if device.index is None:
-        device = torch.device("cuda", torch.cuda.current_device())
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
-    return int(_WS[key][4].item()) if key in _WS else 0
+    ws = _lib.host().workspace_if_any(_device_index(device))
+    return 0 if ws is None else int(ws[4].item())
 
 
 def _stream(device=None):
@@ -75,30 +67,10 @@ def _stream(device=None):
     return torch.cuda.current_stream(device).cuda_stream
 
 
-def _as_bf16_rows(t):
-    if t.dim() != 2:
-        raise ValueError("expected a 2-D tensor")
-    if not t.is_cuda:
-        raise _lib.NVFP4Error("the NVFP4 quantizer runs on a CUDA device only (no CPU path)")
-    x = t if t.dtype == torch.bfloat16 else t.to(torch.bfloat16)
-    if x.stride(1) != 1 or x.stride(0) % 8 != 0 or x.stride(0) < x.shape[1] or x.data_ptr() % 16 != 0:
-        x = x.contiguous()
-    return x
-
-
 def tensor_amax(t, rht=False, signs=None, transpose=False, out=None):
     """Per-tensor |x| maximum of a 2-D tensor as a 1-element fp32 CUDA tensor (after the Hadamard
     transform of its 16-blocks when rht).  No host synchronisation."""
-    x = _as_bf16_rows(t)
-    amax = out if out is not None else torch.empty(1, device=x.device, dtype=torch.float32)
-    sg = _signs(signs, x.device) if rht else None
-    dev = _lib.cuda_device_of(x, amax, sg)
-    with torch.cuda.device(dev):                   # the C side launches on the current device
-        code = _lib.lib().nvfp4_amax_bf16(x.data_ptr(), x.shape[0], x.shape[1], x.stride(0), int(rht),
-                                          int(transpose), sg.data_ptr() if rht else None,
-                                          amax.data_ptr(), 1, _stream(dev))
-    _lib.check(code, "nvfp4_amax_bf16")
-    return amax
+    return _lib.host().amax(t, bool(rht), signs, bool(transpose), out)
 
 
 def quant_nvfp4(t, stochastic=False, rht=False, H=None, signs=None, seed=None, *,
@@ -121,39 +93,10 @@ def quant_nvfp4(t, stochastic=False, rht=False, H=None, signs=None, seed=None, *
         if stochastic:
             _SEED[0] += 1
     _check_h(H)
-    x = _as_bf16_rows(t)
-    rows, cols = x.shape
-    m, k = (cols, rows) if transpose else (rows, cols)
-    if k % BLK != 0:
-        raise AssertionError(f"K={k} must be divisible by {BLK}")
-    dev = x.device
-    sg = _signs(signs, dev) if rht else None
-    sm, sk = swizzled_scale_dims(m, k)
-    qdata = torch.empty((m, k // 2), dtype=torch.uint8, device=dev)
-    scale = torch.empty((sm, sk), dtype=torch.uint8, device=dev)
-    pts = torch.empty((), dtype=torch.float32, device=dev)
-    _lib.cuda_device_of(x, sg, amax)
-    if fused and amax is None and not transpose and rows * (cols // BLK) < 2 ** 31:
-        with torch.cuda.device(dev):               # the C side launches on the current device
-            ws = _workspace(dev)
-            code = _lib.lib().nvfp4_quantize_fused_bf16(
-                x.data_ptr(), rows, cols, x.stride(0),
-                _lib.ROUND_STOCHASTIC if stochastic else _lib.ROUND_NEAREST, int(rht),
-                sg.data_ptr() if rht else None, int(seed) & (2 ** 64 - 1), int(philox_offset),
-                qdata.data_ptr(), scale.data_ptr(), pts.data_ptr(), ws.data_ptr(), 64, _stream(dev))
-        _lib.check(code, "nvfp4_quantize_fused_bf16")
-        return NVFP4Tensor(qdata, scale.view(torch.float8_e4m3fn), BLK, t.dtype, pts, True)
-    if amax is None:
-        amax = tensor_amax(x, rht, sg, transpose)
-    pitch, base = (k // BLK, 0) if counter is None else (int(counter[0]), int(counter[1]))
-    with torch.cuda.device(dev):
-        code = _lib.lib().nvfp4_quantize_shard_bf16(
-            x.data_ptr(), rows, cols, x.stride(0), int(transpose),
-            _lib.ROUND_STOCHASTIC if stochastic else _lib.ROUND_NEAREST, int(rht),
-            sg.data_ptr() if rht else None, amax.data_ptr(), int(seed) & (2 ** 64 - 1), int(philox_offset),
-            pitch, base, qdata.data_ptr(), scale.data_ptr(), pts.data_ptr(), _stream(dev))
-    _lib.check(code, "nvfp4_quantize_shard_bf16")
-    return NVFP4Tensor(qdata, scale.view(torch.float8_e4m3fn), BLK, t.dtype, pts, True)
+    pitch, base = (-1, 0) if counter is None else (int(counter[0]), int(counter[1]))
+    q, s, pts = _lib.host().quantize(t, bool(stochastic), bool(rht), signs, int(seed) & (2 ** 64 - 1), bool(transpose),
+                                     amax, int(philox_offset), bool(fused), pitch, base)
+    return NVFP4Tensor(q, s, BLK, t.dtype, pts, True)
 
 
 def quant_weight_nvfp4(w, amax=None, two_d=False):
@@ -161,42 +104,14 @@ def quant_weight_nvfp4(w, amax=None, two_d=False):
     operands FP4Linear needs (nvfp4_train.py:72-78).  two_d=True scales 16 x 16 tiles (the simulator's
     weight scaling, nvfp4_validate.py:68-82), so that both layouts dequantize to the same matrix.
     amax: optional 1-element fp32 CUDA tensor (a sharded weight passes the group-reduced maximum)."""
-    x = _as_bf16_rows(w)
-    rows, cols = x.shape
-    if rows % BLK != 0 or cols % BLK != 0:
-        raise AssertionError(f"weight dims {rows}x{cols} must be divisible by {BLK}")
-    dev = x.device
-    if amax is None:
-        amax = tensor_amax(x)
-    _lib.cuda_device_of(x, amax)
-    sm_r, sk_r = swizzled_scale_dims(rows, cols)
-    sm_c, sk_c = swizzled_scale_dims(cols, rows)
-    q_r = torch.empty((rows, cols // 2), dtype=torch.uint8, device=dev)
-    s_r = torch.empty((sm_r, sk_r), dtype=torch.uint8, device=dev)
-    q_c = torch.empty((cols, rows // 2), dtype=torch.uint8, device=dev)
-    s_c = torch.empty((sm_c, sk_c), dtype=torch.uint8, device=dev)
-    pts = torch.empty((), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        code = _lib.lib().nvfp4_quantize_weight_bf16(x.data_ptr(), rows, cols, x.stride(0), int(two_d), amax.data_ptr(),
-                                                     q_r.data_ptr(), s_r.data_ptr(), q_c.data_ptr(), s_c.data_ptr(),
-                                                     pts.data_ptr(), _stream(dev))
-    _lib.check(code, "nvfp4_quantize_weight_bf16")
-    return (NVFP4Tensor(q_r, s_r.view(torch.float8_e4m3fn), BLK, w.dtype, pts, True),
-            NVFP4Tensor(q_c, s_c.view(torch.float8_e4m3fn), BLK, w.dtype, pts, True))
+    q_r, s_r, q_c, s_c, pts = _lib.host().quantize_weight(w, amax, bool(two_d))
+    return (NVFP4Tensor(q_r, s_r, BLK, w.dtype, pts, True), NVFP4Tensor(q_c, s_c, BLK, w.dtype, pts, True))
 
 
 def tensor_amax_both(t, signs):
     """fp32 [2] = (max|t|, max|RHT_rows(t)|) from one read of t [rows, cols] (rows % 16 == 0): what
     tensor_amax(t) and tensor_amax(t, True, signs, transpose=True) find in two."""
-    x = _as_bf16_rows(t)
-    sg = _signs(signs, x.device)
-    dev = _lib.cuda_device_of(x, sg)
-    maxima = torch.empty(2, device=dev, dtype=torch.float32)
-    with torch.cuda.device(dev):
-        code = _lib.lib().nvfp4_amax_both_bf16(x.data_ptr(), x.shape[0], x.shape[1], x.stride(0), sg.data_ptr(),
-                                               maxima.data_ptr(), 1, _stream(dev))
-    _lib.check(code, "nvfp4_amax_both_bf16")
-    return maxima
+    return _lib.host().amax_both(t, signs)
 
 
 def quant_dual_nvfp4(t, signs, amax_rows=None, amax_cols=None, stochastic_rows=False, stochastic_cols=False,
@@ -216,42 +131,10 @@ def quant_dual_nvfp4(t, signs, amax_rows=None, amax_cols=None, stochastic_rows=F
         seed_cols = _SEED[0]
         if stochastic_cols:
             _SEED[0] += 1
-    x = _as_bf16_rows(t)
-    rows, cols = x.shape
-    if rows % BLK != 0 or cols % BLK != 0:
-        raise AssertionError(f"dims {rows}x{cols} must be divisible by {BLK}")
-    dev = x.device
-    sg = _signs(signs, dev)
-    if amax_rows is None and amax_cols is None:
-        both = tensor_amax_both(x, sg)
-        amax_rows, amax_cols = both[0:1], both[1:2]
-    elif amax_cols is None:
-        amax_cols = tensor_amax(x, True, sg, transpose=True)
-    elif amax_rows is None:
-        amax_rows = tensor_amax(x)
-    _lib.cuda_device_of(x, sg, amax_rows, amax_cols)
-    sm_r, sk_r = swizzled_scale_dims(rows, cols)
-    sm_c, sk_c = swizzled_scale_dims(cols, rows)
-    q_r = torch.empty((rows, cols // 2), dtype=torch.uint8, device=dev)
-    s_r = torch.empty((sm_r, sk_r), dtype=torch.uint8, device=dev)
-    q_c = torch.empty((cols, rows // 2), dtype=torch.uint8, device=dev)
-    s_c = torch.empty((sm_c, sk_c), dtype=torch.uint8, device=dev)
-    pts_r = torch.empty((), dtype=torch.float32, device=dev)
-    pts_c = torch.empty((), dtype=torch.float32, device=dev)
-    ctr = None
-    if counters is not None:
-        import ctypes
-        ctr = (ctypes.c_uint64 * 4)(*[int(v) for v in counters])
-    mode = lambda sr: _lib.ROUND_STOCHASTIC if sr else _lib.ROUND_NEAREST
-    with torch.cuda.device(dev):
-        code = _lib.lib().nvfp4_quantize_dual_bf16(
-            x.data_ptr(), rows, cols, x.stride(0), mode(stochastic_rows), mode(stochastic_cols), sg.data_ptr(),
-            amax_rows.data_ptr(), amax_cols.data_ptr(), int(seed_rows) & (2 ** 64 - 1), int(seed_cols) & (2 ** 64 - 1),
-            int(philox_offset), ctr, q_r.data_ptr(), s_r.data_ptr(), pts_r.data_ptr(), q_c.data_ptr(), s_c.data_ptr(),
-            pts_c.data_ptr(), _stream(dev))
-    _lib.check(code, "nvfp4_quantize_dual_bf16")
-    return (NVFP4Tensor(q_r, s_r.view(torch.float8_e4m3fn), BLK, t.dtype, pts_r, True),
-            NVFP4Tensor(q_c, s_c.view(torch.float8_e4m3fn), BLK, t.dtype, pts_c, True))
+    q_r, s_r, p_r, q_c, s_c, p_c = _lib.host().quantize_dual(
+        t, signs, amax_rows, amax_cols, bool(stochastic_rows), bool(stochastic_cols), int(seed_rows) & (2 ** 64 - 1),
+        int(seed_cols) & (2 ** 64 - 1), int(philox_offset), [] if counters is None else [int(v) for v in counters])
+    return (NVFP4Tensor(q_r, s_r, BLK, t.dtype, p_r, True), NVFP4Tensor(q_c, s_c, BLK, t.dtype, p_c, True))
 
 
 # the reference's second name for the same entry (nvfp4_cuda.py:158)
