@@ -61,14 +61,6 @@ static Choice choose(int64_t M, int64_t N, int64_t K, int forced, bool may_split
   const int64_t slices = (K + 255) / 256;
   Choice best{true, 256, 1};
   float best_us = 3.0e38f;
-#ifdef NVFP4_TUNE
-  if (const char* e = getenv("NVFP4_TUNE")) {
-    int v = atoi(e), sp = 1;
-    if (const char* c = strchr(e, ',')) sp = atoi(c + 1);
-    if ((slices + sp - 1) / sp * (sp - 1) >= slices) sp = 1;
-    return Choice{v < 0, v < 0 ? -v : v, sp};
-  }
-#endif
   for (const Kind& k : kinds) {
     if (forced != 0 && k.pair != (forced == 2)) continue;
     const int64_t rows = k.pair ? 256 : 128, tiles = ((M + rows - 1) / rows) * ((N + k.tile_n - 1) / k.tile_n);
