@@ -23,7 +23,7 @@ namespace {
 
 #define NVFP4_FOR_EACH(F)                                                                                              \
   F(nvfp4_amax_bf16) F(nvfp4_amax_both_bf16) F(nvfp4_quantize_fused_bf16) F(nvfp4_quantize_shard_bf16)                 \
-  F(nvfp4_quantize_weight_bf16) F(nvfp4_quantize_dual_bf16) F(nvfp4_gemm) F(nvfp4_gemm_amax)
+  F(nvfp4_quantize_weight_bf16) F(nvfp4_quantize_dual_bf16) F(nvfp4_round_amax_f32) F(nvfp4_gemm) F(nvfp4_gemm_amax)
 
 struct Library {
 #define F(name) decltype(&::name) name = nullptr;
@@ -155,6 +155,24 @@ at::Tensor as_bf16_rows(const at::Tensor& t) {
   return as_rows(t.scalar_type() == at::kBFloat16 ? t : t.to(at::kBFloat16), 8);
 }
 
+// An fp32 matrix whose bf16 rounding and maximum (both maxima with signs: after the Hadamard transform along the rows
+// too) one kernel finds: (bf16 copy, maxima).  For shapes that the kernel takes.
+bool can_round(const at::Tensor& t, bool rht) {
+  return t.scalar_type() == at::kFloat && t.size(0) > 0 && t.size(1) > 0 && t.size(1) % 8 == 0 &&
+         (!rht || t.size(0) % 16 == 0) && t.size(0) <= 64 * 65535LL;
+}
+std::pair<at::Tensor, at::Tensor> round_amax(const at::Tensor& t, const at::Tensor* signs) {
+  const at::Tensor x = as_rows(t, 4);
+  const c10::Device dev = device_of({&x, signs});
+  at::Tensor out = at::empty({x.size(0), x.size(1)}, on(dev, at::kBFloat16));
+  at::Tensor maxima = at::empty({signs != nullptr ? 2 : 1}, on(dev, at::kFloat));
+  check(lib.nvfp4_round_amax_f32(static_cast<const float*>(x.data_ptr()), x.size(0), x.size(1), x.stride(0), out.data_ptr(),
+                                 signs != nullptr ? static_cast<const float*>(signs->data_ptr()) : nullptr,
+                                 static_cast<float*>(maxima.data_ptr()), 1, stream_of(dev)),
+        "nvfp4_round_amax_f32");
+  return {out, maxima};
+}
+
 struct Operand {
   at::Tensor q, s, p;
   uint8_t* qp() { return q.data_ptr<uint8_t>(); }
@@ -210,23 +228,30 @@ py::tuple quantize(const at::Tensor& t, bool stochastic, bool rht, const OptTens
                    const OptTensor& amax_in, uint64_t offset, bool fused, int64_t counter_pitch, int64_t counter_base) {
   check_matrix(t);
   const c10::cuda::CUDAGuard guard(t.device());
-  const at::Tensor x = as_bf16_rows(t);
+  // fp32 without a known maximum: the rounding finds it on the way.  Row-wise the single-launch kernel needs no pass of
+  // its own for it, so there this pays only from 4M elements on (one read of the bf16 copy against one more launch).
+  at::Tensor x, found;
+  if (!amax_in.has_value() && !rht && fused && can_round(t, false) && (transpose || t.numel() >= (1 << 22)))
+    std::tie(x, found) = round_amax(t, nullptr);
+  else
+    x = as_bf16_rows(t);
+  const at::Tensor* known = amax_in.has_value() ? &*amax_in : (found.defined() ? &found : nullptr);
   const int64_t rows = x.size(0), cols = x.size(1), m = transpose ? cols : rows, k = transpose ? rows : cols;
   if (k % 16 != 0) raise(PyExc_AssertionError, "K=" + std::to_string(k) + " must be divisible by 16");
   at::Tensor sg;
   if (rht) sg = signs_on(signs, x.device());
-  const c10::Device dev = device_of({&x, rht ? &sg : nullptr, ptr_of(amax_in)});
+  const c10::Device dev = device_of({&x, rht ? &sg : nullptr, known});
   Operand o = alloc(dev, m, k);
   void* stream = stream_of(dev);
   const float* sgp = rht ? float_ptr(sg) : nullptr;
-  if (fused && !amax_in.has_value() && !transpose && rows * (cols / 16) < (1LL << 31)) {
+  if (fused && known == nullptr && !transpose && rows * (cols / 16) < (1LL << 31)) {
     at::Tensor ws = workspace(dev.index());
     check(lib.nvfp4_quantize_fused_bf16(x.data_ptr(), rows, cols, x.stride(0), stochastic, rht, sgp, seed, offset, o.qp(),
                                         o.sp(), o.pp(), ws.data_ptr(), 64, stream),
           "nvfp4_quantize_fused_bf16");
     return py::make_tuple(o.q, o.s, o.p);
   }
-  const at::Tensor a = amax_in.has_value() ? *amax_in : amax_rows(x, rht, rht ? &sg : nullptr, transpose, OptTensor());
+  const at::Tensor a = known != nullptr ? *known : amax_rows(x, rht, rht ? &sg : nullptr, transpose, OptTensor());
   const uint64_t pitch = counter_pitch < 0 ? (uint64_t)(k / 16) : (uint64_t)counter_pitch;
   check(lib.nvfp4_quantize_shard_bf16(x.data_ptr(), rows, cols, x.stride(0), transpose, stochastic, rht, sgp, float_ptr(a),
                                       seed, offset, pitch, counter_pitch < 0 ? 0 : (uint64_t)counter_base, o.qp(), o.sp(),
@@ -239,11 +264,14 @@ py::tuple quantize(const at::Tensor& t, bool stochastic, bool rht, const OptTens
 py::tuple quantize_weight(const at::Tensor& w, const OptTensor& amax_in, bool two_d) {
   check_matrix(w);
   const c10::cuda::CUDAGuard guard(w.device());
-  const at::Tensor x = as_bf16_rows(w);
+  at::Tensor x, a;
+  if (!amax_in.has_value() && can_round(w, false)) std::tie(x, a) = round_amax(w, nullptr);
+  else x = as_bf16_rows(w);
   const int64_t rows = x.size(0), cols = x.size(1);
   if (rows % 16 != 0 || cols % 16 != 0)
     raise(PyExc_AssertionError, "weight dims " + std::to_string(rows) + "x" + std::to_string(cols) + " must be divisible by 16");
-  const at::Tensor a = amax_in.has_value() ? *amax_in : amax_rows(x, false, nullptr, false, OptTensor());
+  if (amax_in.has_value()) a = *amax_in;
+  else if (!a.defined()) a = amax_rows(x, false, nullptr, false, OptTensor());
   const c10::Device dev = device_of({&x, &a});
   Operand r = alloc(dev, rows, cols), c = alloc(dev, cols, rows, false);
   check(lib.nvfp4_quantize_weight_bf16(x.data_ptr(), rows, cols, x.stride(0), two_d, float_ptr(a), r.qp(), r.sp(), c.qp(),
@@ -258,15 +286,17 @@ py::tuple quantize_dual(const at::Tensor& t, const OptTensor& signs, const OptTe
                         const std::vector<uint64_t>& counters) {
   check_matrix(t);
   const c10::cuda::CUDAGuard guard(t.device());
-  const at::Tensor x = as_bf16_rows(t);
-  const int64_t rows = x.size(0), cols = x.size(1);
+  const int64_t rows = t.size(0), cols = t.size(1);
   if (rows % 16 != 0 || cols % 16 != 0)
     raise(PyExc_AssertionError, "dims " + std::to_string(rows) + "x" + std::to_string(cols) + " must be divisible by 16");
-  const at::Tensor sg = signs_on(signs, x.device());
-  at::Tensor r, c, both;                                     // `both` keeps the two words alive past the launch
+  const at::Tensor sg = signs_on(signs, t.device());
+  at::Tensor x, r, c, both;                                  // `both`: the two maxima found here
   if (amax_r.has_value()) r = *amax_r;
   if (amax_c.has_value()) c = *amax_c;
-  if (!r.defined() && !c.defined()) both = amax_both_rows(x, sg);
+  if (!r.defined() && !c.defined() && can_round(t, true)) std::tie(x, both) = round_amax(t, &sg);
+  else x = as_bf16_rows(t);
+  if (both.defined()) {}
+  else if (!r.defined() && !c.defined()) both = amax_both_rows(x, sg);
   else if (!c.defined()) c = amax_rows(x, true, &sg, true, OptTensor());
   else if (!r.defined()) r = amax_rows(x, false, nullptr, false, OptTensor());
   const c10::Device dev = device_of({&x, &sg, r.defined() ? &r : nullptr, c.defined() ? &c : nullptr});

@@ -155,6 +155,49 @@ __global__ void __launch_bounds__(512) amax_plain_kernel(const uint16_t* __restr
   cta_max_to(amax, __uint_as_float(m << 16));
 }
 
+// eight fp32 values -> eight packed bf16, round to nearest even
+__device__ __forceinline__ uint4 round8(const float4& a, const float4& b) {
+  auto pack = [](float lo, float hi) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  };
+  return make_uint4(pack(a.x, a.y), pack(a.z, a.w), pack(b.x, b.y), pack(b.z, b.w));
+}
+
+// fp32 -> bf16 copy (contiguous rows) and the plain maximum of the copy in one pass of 6 bytes per element, where a
+// cast and amax_plain_kernel move 8.  HBM-bound; two 32-byte reads per thread in flight.
+__global__ void __launch_bounds__(512) round_amax_kernel(const float* __restrict__ x, int64_t rows, int vec_per_row,
+                                                         int64_t ld, uint16_t* __restrict__ out,
+                                                         float* __restrict__ amax) {
+  const int64_t total = rows * vec_per_row, stride = (int64_t)gridDim.x * blockDim.x;
+  const bool flat = ld == (int64_t)vec_per_row * 8;
+  uint32_t m = 0;
+  auto src = [&](int64_t i) {
+    if (flat) return reinterpret_cast<const float4*>(x) + 2 * i;
+    const int64_t r = i / vec_per_row;
+    return reinterpret_cast<const float4*>(x + r * ld) + 2 * (i - r * vec_per_row);
+  };
+  auto fold = [&](int64_t i, const float4& a, const float4& b) {
+    const uint32_t k = 0x7fff7fffu;
+    const uint4 q = round8(a, b);
+    reinterpret_cast<uint4*>(out)[i] = q;
+    m = __vimax3_u16x2(__vimax3_u16x2(q.x & k, q.y & k, q.z & k), q.w & k, m);
+  };
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + stride < total; i += 2 * stride) {
+    const float4 *p = src(i), *q = src(i + stride);
+    const float4 a0 = __ldg(p), b0 = __ldg(p + 1), a1 = __ldg(q), b1 = __ldg(q + 1);
+    fold(i, a0, b0);
+    fold(i + stride, a1, b1);
+  }
+  if (i < total) {
+    const float4* p = src(i);
+    fold(i, __ldg(p), __ldg(p + 1));
+  }
+  m = max(m & 0xffffu, m >> 16);
+  cta_max_to(amax, __uint_as_float(m << 16));
+}
+
 // maximum after the Hadamard transform, blocks along the columns: one thread per block
 __global__ void __launch_bounds__(256) amax_rht_rows_kernel(const uint16_t* __restrict__ x,
                                                             int64_t rows, int blk_per_row, int64_t ld,
@@ -344,11 +387,36 @@ __device__ __forceinline__ void wide_stage(uint32_t* tile, const WideTile& t, co
   for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(&tile[(4 * k + t.lr) * kWidePitch + (t.cc >> 1)]) = d[k];
 }
 
-// BOTH: maxima2[0] = plain maximum as well (else only maxima2[0] = maximum after the transform)
-template <bool BOTH>
-__global__ void __launch_bounds__(256) amax_cols_wide_kernel(const uint16_t* __restrict__ x, int64_t rows, int64_t cols,
+// The same tile out of an fp32 matrix, rounded to bf16 on the way (and written to `out`, contiguous rows).
+__device__ __forceinline__ void wide_fetch_round(const float* __restrict__ x, int64_t rows, int64_t cols, int64_t ld,
+                                                 const WideTile& t, int j, uint16_t* __restrict__ out, uint4 (&d)[4]) {
+  float4 a[4], b[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int64_t r = t.r_base + 16 * j + 4 * k + t.lr;
+    const bool in = t.col_in && r < rows;
+    const float4* p = reinterpret_cast<const float4*>(x + r * ld + t.c0 + t.cc);
+    a[k] = in ? __ldg(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+    b[k] = in ? __ldg(p + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int64_t r = t.r_base + 16 * j + 4 * k + t.lr;
+    d[k] = round8(a[k], b[k]);
+    if (t.col_in && r < rows) *reinterpret_cast<uint4*>(out + r * cols + t.c0 + t.cc) = d[k];
+  }
+}
+
+// BOTH: maxima2[0] = plain maximum as well (else only maxima2[0] = maximum after the transform).  F32: x is fp32, the
+// maxima are those of its bf16 rounding, which goes to `rounded`.
+template <bool BOTH, bool F32>
+__global__ void __launch_bounds__(256) amax_cols_wide_kernel(const void* __restrict__ x, int64_t rows, int64_t cols,
                                                              int64_t ld, const float* __restrict__ signs16,
-                                                             float* __restrict__ out) {
+                                                             float* __restrict__ out, uint16_t* __restrict__ rounded) {
+  auto fetch = [&](const WideTile& t, int j, uint4 (&d)[4]) {
+    if (F32) wide_fetch_round(static_cast<const float*>(x), rows, cols, ld, t, j, rounded, d);
+    else wide_fetch(static_cast<const uint16_t*>(x), rows, ld, t, j, d);
+  };
   __shared__ __align__(16) uint32_t tile[16 * kWidePitch];
   float sg[16];
   load_signs(signs16, sg);
@@ -358,7 +426,7 @@ __global__ void __launch_bounds__(256) amax_cols_wide_kernel(const uint16_t* __r
   float m = 0.0f;
   uint32_t mp = 0u;
   uint4 nxt[4];
-  wide_fetch(x, rows, ld, t, 0, nxt);
+  fetch(t, 0, nxt);
 #pragma unroll 1
   for (int j = 0; j < 4; ++j) {
     if (t.r_base + 16 * j >= rows) break;                  // uniform over the CTA
@@ -371,7 +439,7 @@ __global__ void __launch_bounds__(256) amax_cols_wide_kernel(const uint16_t* __r
         mp = __vimax3_u16x2(mp, nxt[k].z & kk, nxt[k].w & kk);
       }
     }
-    if (j + 1 < 4) wide_fetch(x, rows, ld, t, j + 1, nxt);
+    if (j + 1 < 4) fetch(t, j + 1, nxt);
     __syncthreads();
     if (t.mine) {
       float v0[16], v1[16];
@@ -543,7 +611,7 @@ extern "C" int nvfp4_amax_bf16(const void* x, int64_t rows, int64_t cols, int64_
     if (grid.y > 65535u) return NVFP4_E_SHAPE;
     if ((cols & 7) == 0) {
       const dim3 wgrid((unsigned)((cols + kWideCols - 1) / kWideCols), grid.y);
-      amax_cols_wide_kernel<false><<<wgrid, 256, 0, stream>>>(xp, rows, cols, ld, signs16, amax);
+      amax_cols_wide_kernel<false, false><<<wgrid, 256, 0, stream>>>(xp, rows, cols, ld, signs16, amax, nullptr);
     } else {
       amax_rht_cols_kernel<<<grid, 256, 0, stream>>>(xp, rows, cols, ld, signs16, amax);
     }
@@ -650,9 +718,30 @@ extern "C" int nvfp4_amax_both_bf16(const void* x, int64_t rows, int64_t cols, i
   if (grid.y > 65535u) return NVFP4_E_LIMIT;
   if ((cols & 7) == 0) {
     const dim3 wgrid((unsigned)((cols + kWideCols - 1) / kWideCols), grid.y);
-    amax_cols_wide_kernel<true><<<wgrid, 256, 0, stream>>>(static_cast<const uint16_t*>(x), rows, cols, ld, signs16, maxima2);
+    amax_cols_wide_kernel<true, false><<<wgrid, 256, 0, stream>>>(x, rows, cols, ld, signs16, maxima2, nullptr);
   } else {
     amax_both_cols_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(x), rows, cols, ld, signs16, maxima2);
+  }
+  return cudaGetLastError() == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
+}
+
+extern "C" int nvfp4_round_amax_f32(const float* x, int64_t rows, int64_t cols, int64_t ld, void* out_bf16,
+                                    const float* signs16, float* maxima, int zero_first, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (!x || !out_bf16 || !maxima) return NVFP4_E_NULL;
+  if (rows <= 0 || cols <= 0 || ld < cols || (cols & 7) != 0 || (signs16 != nullptr && (rows & 15) != 0)) return NVFP4_E_SHAPE;
+  if (!aligned16(x) || (ld & 3) != 0 || !aligned16(out_bf16) || (signs16 != nullptr && !aligned16(signs16)))
+    return NVFP4_E_ALIGN;
+  if ((rows + 63) / 64 > 65535 || cols / 8 > 0x7fffffffLL) return NVFP4_E_LIMIT;
+  const size_t words = signs16 != nullptr ? 2 : 1;
+  if (zero_first && cudaMemsetAsync(maxima, 0, words * sizeof(float), stream) != cudaSuccess) return NVFP4_E_LAUNCH;
+  uint16_t* out = static_cast<uint16_t*>(out_bf16);
+  if (signs16 != nullptr) {
+    const dim3 grid((unsigned)((cols + kWideCols - 1) / kWideCols), (unsigned)((rows + 63) / 64));
+    amax_cols_wide_kernel<true, true><<<grid, 256, 0, stream>>>(x, rows, cols, ld, signs16, maxima, out);
+  } else {
+    const int vpr = (int)(cols >> 3);
+    round_amax_kernel<<<grid_for(rows * vpr, 512 * 2, 148 * 4), 512, 0, stream>>>(x, rows, vpr, ld, out, maxima);
   }
   return cudaGetLastError() == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
 }

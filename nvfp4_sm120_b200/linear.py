@@ -263,11 +263,11 @@ class WeightQuantCache:
         if not _AMORTIZE:
             return None, None
         if self.step != _STEP[0]:
-            w = weight.detach()
-            if w.dtype != torch.bfloat16:
-                w = w.to(torch.bfloat16)          # one cast of the fp32 master weight serves all three kernels
-            amax = tensor_amax(w)
-            if amax_reduce is not None:
+            w, amax = weight.detach(), None
+            if amax_reduce is not None:           # (without it the rounding to bf16 finds the maximum on the way)
+                if w.dtype != torch.bfloat16:
+                    w = w.to(torch.bfloat16)      # one cast of the fp32 master weight serves all three kernels
+                amax = tensor_amax(w)
                 amax_reduce(amax)
             # [N, K] with contraction K (fprop) and [K, N] with contraction N (dgrad)
             self.wq_K, self.wq_N = quant_weight_nvfp4(w, amax=amax, two_d=self.two_d)
