@@ -167,6 +167,15 @@ int nvfp4_quantize_dual_bf16(const void* x, int64_t rows, int64_t cols, int64_t 
                              uint8_t* qdata_cols, uint8_t* scales_cols, float* pts_cols, void* stream);
 
 /*
+ * out_bf16[rows, cols] (contiguous) = x rounded to bf16 (nearest even) and the maxima of that copy, from one read of
+ * x[rows, cols] (fp32, row stride ld): maxima[0] = max|.|, and with signs16 also maxima[1] = the maximum after the
+ * Hadamard transform along the rows (the words of nvfp4_amax_both_bf16; rows % 16 == 0).  cols % 8 == 0, ld % 4 == 0,
+ * 16-byte aligned pointers.  The reference casts an fp32 operand first and reads the copy again for its maximum.
+ */
+int nvfp4_round_amax_f32(const float* x, int64_t rows, int64_t cols, int64_t ld, void* out_bf16, const float* signs16,
+                         float* maxima, int zero_first, void* stream);
+
+/*
  * maxima2[0] = max|x| and maxima2[1] = max|RHT_rows(x)| (16-point random-sign Hadamard over groups
  * of 16 rows) from one read of x[rows, cols]; rows % 16 == 0, cols even.  The two words are what
  * nvfp4_amax_bf16 gives with (rht 0) and with (rht 1, transpose 1).
@@ -325,6 +334,17 @@ int nvfp4_rmsnorm_fwd(const void* x, int x_is_f32, const float* weight, int64_t 
 int nvfp4_rmsnorm_bwd(const void* x, int x_is_f32, const float* weight, const float* rstd, const void* g,
                       int g_is_f32, int64_t rows, int64_t cols, void* dx, float* dweight, int zero_first,
                       void* stream);
+
+/*
+ * Rotary position embedding of q and k (bf16, contiguous [rows, heads * head_dim], row r = position r % seq): with a, b
+ * the halves of a head, a' = a cos - b sin, b' = b cos + a sin, fp32 products and sums, one rounding to bf16.  backward != 0:
+ * the gradient of that, a = ga' cos + gb' sin, b = gb' cos - ga' sin, every product rounded to bf16 as autograd does.
+ * cosine / sine: fp32 [seq, head_dim / 2].  head_dim % 16 == 0, 16-byte aligned pointers, rows % seq == 0.  The torch
+ * operations of nvfp4_train.py:91-98 on both tensors, bit for bit.
+ */
+int nvfp4_rotary_bf16(const void* q, void* q_out, int q_heads, const void* k, void* k_out, int k_heads, int64_t rows,
+                      int64_t seq, int head_dim, const float* cosine, const float* sine, int backward, void* stream);
+
 
 /*
  * Test hooks of the bounded waits, process-wide, for the launches that follow.  Every spin inside

@@ -13,6 +13,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import rotary
 from .linear import FP4Linear, make_linear
 from .norm import rmsnorm_amax
 from .swiglu import relu2
@@ -99,8 +100,13 @@ class DecoderBlock(nn.Module):
                 q, k, v = self.q(h, **kw), self.k(h, **kw), self.v(h, **kw)
         else:
             q, k, v = self.q(h), self.k(h), self.v(h)
-        q, k, v = split(q, self.n_heads), split(k, self.n_kv), split(v, self.n_kv)
-        q, k = apply_rotary(q, cos, sin), apply_rotary(k, cos, sin)
+        heads = lambda t, n: t.view(B, T, n, self.head_dim)
+        if rotary.takes(heads(q, self.n_heads), heads(k, self.n_kv), cos, sin):
+            q, k = rotary.rotary(heads(q, self.n_heads), heads(k, self.n_kv), cos, sin)
+            q, k, v = q.transpose(1, 2), k.transpose(1, 2), split(v, self.n_kv)
+        else:
+            q, k, v = split(q, self.n_heads), split(k, self.n_kv), split(v, self.n_kv)
+            q, k = apply_rotary(q, cos, sin), apply_rotary(k, cos, sin)
         if self.n_kv != self.n_heads:
             rep = self.n_heads // self.n_kv
             k, v = k.repeat_interleave(rep, 1), v.repeat_interleave(rep, 1)
