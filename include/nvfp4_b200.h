@@ -271,6 +271,15 @@ int nvfp4_gemm_fp4out(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pt
 int nvfp4_gemm_set_mode(int mode);
 
 /*
+ * nvfp4_gemm with a bf16 result held in fp32: D = float(bf16(A B^T)), what nvfp4_gemm(NVFP4_OUT_BF16) and a cast give,
+ * without the bf16 tensor in memory and the pass over it.  For fp32 activations: the reference's FP4Linear returns
+ * its bf16 product in the activation's dtype (nvfp4_train.py:36-55).
+ */
+int nvfp4_gemm_bf16_as_f32(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pts, const uint8_t* b_q,
+                           const uint8_t* b_sf, const float* b_pts, float* d, int64_t M, int64_t N, int64_t K, int64_t ldd,
+                           int32_t* status, void* stream);
+
+/*
  * Producer fusion in front of the quantizer: SwiGLU and its backward in one pass each that also
  * leaves the per-tensor maxima the following quantizations need, so that those run as one
  * nvfp4_quantize_bf16 call with the amax given (no separate amax pass).

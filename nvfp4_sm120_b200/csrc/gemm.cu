@@ -87,7 +87,9 @@ __device__ __forceinline__ void sum_partials(const Params& p, uint32_t smem_base
       float4 s = v[b][0];
 #pragma unroll
       for (int k = 1; k < S; ++k) { s.x += v[b][k].x; s.y += v[b][k].y; s.z += v[b][k].z; s.w += v[b][k].w; }
-      const float o[4] = {s.x * alpha, s.y * alpha, s.z * alpha, s.w * alpha};
+      float o[4] = {s.x * alpha, s.y * alpha, s.z * alpha, s.w * alpha};
+      if (p.round_bf16)
+        for (int j = 0; j < 4; ++j) o[j] = __bfloat162float(__float2bfloat16_rn(o[j]));
       const int64_t d = (m0 + r) * p.ldd + col;
       const bool vec = col + 4 <= p.N && (p.ldd & 3) == 0;
       if (p.out_f32) {

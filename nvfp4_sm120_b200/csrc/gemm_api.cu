@@ -80,7 +80,7 @@ static Choice choose(int64_t M, int64_t N, int64_t K, int forced, bool may_split
 static int gemm_any(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pts, const uint8_t* b_q,
                     const uint8_t* b_sf, const float* b_pts, void* d, int out_dtype, int64_t M, int64_t N,
                     int64_t K, int64_t ldd, uint8_t* d_sf, const float* d_amax, float* d_amax_out, int32_t* status,
-                    void* stream_) {
+                    void* stream_, int round_bf16 = 0) {
   using namespace nvfp4::gemm;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const bool fp4_out = d_sf != nullptr;
@@ -99,7 +99,7 @@ static int gemm_any(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pts,
   const Choice pick = choose(M, N, K, forced, !fp4_out && d_amax_out == nullptr);
   Params p{a_sf, b_sf, a_pts, b_pts, d, M, N, K, ldd, out_dtype == NVFP4_OUT_F32 ? 1 : 0, status, pick.splits, 0,
            g_gemm_wait_ns.load(std::memory_order_relaxed), g_gemm_drop_arrival.load(std::memory_order_relaxed),
-           d_sf, d_amax, fp4_out ? 1 : 0, d_amax_out};
+           d_sf, d_amax, fp4_out ? 1 : 0, round_bf16, d_amax_out};
   // The epilogue stores through TMA when the row pitch allows a tensor map (a multiple of 16 bytes).
   CUtensorMap map_d{};                                         // unused otherwise
   if (p.splits == 1 && !fp4_out && (ldd * (p.out_f32 ? 4 : 2)) % 16 == 0) {
@@ -115,6 +115,13 @@ extern "C" int nvfp4_gemm(const uint8_t* a_q, const uint8_t* a_sf, const float* 
                           int64_t K, int64_t ldd, int32_t* status, void* stream_) {
   return gemm_any(a_q, a_sf, a_pts, b_q, b_sf, b_pts, d, out_dtype, M, N, K, ldd, nullptr, nullptr, nullptr, status,
                   stream_);
+}
+
+extern "C" int nvfp4_gemm_bf16_as_f32(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pts, const uint8_t* b_q,
+                                      const uint8_t* b_sf, const float* b_pts, float* d, int64_t M, int64_t N, int64_t K,
+                                      int64_t ldd, int32_t* status, void* stream_) {
+  return gemm_any(a_q, a_sf, a_pts, b_q, b_sf, b_pts, d, NVFP4_OUT_F32, M, N, K, ldd, nullptr, nullptr, nullptr, status,
+                  stream_, 1);
 }
 
 extern "C" int nvfp4_gemm_amax(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pts, const uint8_t* b_q,

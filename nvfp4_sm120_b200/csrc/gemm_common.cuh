@@ -163,6 +163,7 @@ struct Params {
   uint8_t* d_sf;                      // swizzled E4M3 scales of the [M, N] operand
   const float* d_amax;
   int out_fp4;
+  int round_bf16;                     // fp32 output holds the result rounded to bf16 (a bf16 product for an fp32 caller)
   // optional: the kernel leaves max|D| over the stored output (after its rounding to the output type) in
   // this zeroed fp32 word, so that a quantizer reading D next needs no pass of its own to find it
   float* d_amax_out;
@@ -220,6 +221,12 @@ __device__ __forceinline__ void quantize_out_block(const uint32_t* acc, float al
        (e2m1x2_rn(v[12] * recip, v[13] * recip) << 16) | (e2m1x2_rn(v[14] * recip, v[15] * recip) << 24);
 }
 
+// one value of an fp32 result
+__device__ __forceinline__ float out_f32(const Params& p, uint32_t acc, float alpha) {
+  const float v = __uint_as_float(acc) * alpha;
+  return p.round_bf16 ? __bfloat162float(__float2bfloat16_rn(v)) : v;
+}
+
 __device__ __forceinline__ void store_row_chunk(const Params& p, int64_t row, int64_t col, const uint32_t (&r)[32],
                                                 float alpha) {
   const bool full = (col + 32 <= p.N);
@@ -247,13 +254,12 @@ __device__ __forceinline__ void store_row_chunk(const Params& p, int64_t row, in
     if (full && ((p.ldd & 3) == 0)) {
 #pragma unroll
       for (int j = 0; j < 32; j += 4)
-        *reinterpret_cast<float4*>(out + j) =
-            make_float4(__uint_as_float(r[j]) * alpha, __uint_as_float(r[j + 1]) * alpha,
-                        __uint_as_float(r[j + 2]) * alpha, __uint_as_float(r[j + 3]) * alpha);
+        *reinterpret_cast<float4*>(out + j) = make_float4(out_f32(p, r[j], alpha), out_f32(p, r[j + 1], alpha),
+                                                          out_f32(p, r[j + 2], alpha), out_f32(p, r[j + 3], alpha));
     } else {
 #pragma unroll
       for (int j = 0; j < 32; ++j)
-        if (col + j < p.N) out[j] = __uint_as_float(r[j]) * alpha;
+        if (col + j < p.N) out[j] = out_f32(p, r[j], alpha);
     }
   } else {
     __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.d) + row * p.ldd + col;
@@ -312,8 +318,8 @@ __device__ __forceinline__ void drain_through_tma(const Params& p, const CUtenso
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         *reinterpret_cast<float4*>(rowp + (((uint32_t)j ^ sw) << 4)) =
-            make_float4(__uint_as_float(r[4 * j]) * alpha, __uint_as_float(r[4 * j + 1]) * alpha,
-                        __uint_as_float(r[4 * j + 2]) * alpha, __uint_as_float(r[4 * j + 3]) * alpha);
+            make_float4(out_f32(p, r[4 * j], alpha), out_f32(p, r[4 * j + 1], alpha), out_f32(p, r[4 * j + 2], alpha),
+                        out_f32(p, r[4 * j + 3], alpha));
     } else {
       const int half = ((c0 - c_begin) >> 5) & 1;
 #pragma unroll

@@ -346,8 +346,8 @@ gemm3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             *reinterpret_cast<float4*>(rowp + (((uint32_t)j ^ sw) << 4)) =
-                make_float4(__uint_as_float(r[4 * j]) * alpha, __uint_as_float(r[4 * j + 1]) * alpha,
-                            __uint_as_float(r[4 * j + 2]) * alpha, __uint_as_float(r[4 * j + 3]) * alpha);
+                make_float4(out_f32(p, r[4 * j], alpha), out_f32(p, r[4 * j + 1], alpha), out_f32(p, r[4 * j + 2], alpha),
+                            out_f32(p, r[4 * j + 3], alpha));
           send_box(col0 + 32 * ch, row0);
         }
       }

@@ -23,7 +23,8 @@ namespace {
 
 #define NVFP4_FOR_EACH(F)                                                                                              \
   F(nvfp4_amax_bf16) F(nvfp4_amax_both_bf16) F(nvfp4_quantize_fused_bf16) F(nvfp4_quantize_shard_bf16)                 \
-  F(nvfp4_quantize_weight_bf16) F(nvfp4_quantize_dual_bf16) F(nvfp4_round_amax_f32) F(nvfp4_gemm) F(nvfp4_gemm_amax)
+  F(nvfp4_quantize_weight_bf16) F(nvfp4_quantize_dual_bf16) F(nvfp4_round_amax_f32) F(nvfp4_gemm) F(nvfp4_gemm_amax) \
+  F(nvfp4_gemm_bf16_as_f32)
 
 struct Library {
 #define F(name) decltype(&::name) name = nullptr;
@@ -328,6 +329,20 @@ at::Tensor mm(const at::Tensor& aq, const at::Tensor& as, const at::Tensor& ap, 
   return d;
 }
 
+// the bf16 product in an fp32 tensor
+at::Tensor mm_bf16_as_f32(const at::Tensor& aq, const at::Tensor& as, const at::Tensor& ap, const at::Tensor& bq,
+                          const at::Tensor& bs, const at::Tensor& bp) {
+  const int64_t m = aq.size(0), k2 = aq.size(1), n = bq.size(0);
+  const c10::Device dev = device_of({&aq, &as, &ap, &bq, &bs, &bp});
+  const c10::cuda::CUDAGuard guard(dev);
+  const at::Tensor d = at::empty({m, n}, on(dev, at::kFloat));
+  auto u8 = [](const at::Tensor& t) { return static_cast<const uint8_t*>(t.data_ptr()); };
+  check(lib.nvfp4_gemm_bf16_as_f32(u8(aq), u8(as), float_ptr(ap), u8(bq), u8(bs), float_ptr(bp), float_ptr(d), m, n, k2 * 2,
+                                   n, status_word(dev.index()).data_ptr<int32_t>(), stream_of(dev)),
+        "nvfp4_gemm_bf16_as_f32");
+  return d;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
@@ -341,4 +356,5 @@ PYBIND11_MODULE(_host, m) {
   m.def("quantize_weight", &quantize_weight);
   m.def("quantize_dual", &quantize_dual);
   m.def("mm", &mm);
+  m.def("mm_bf16_as_f32", &mm_bf16_as_f32);
 }

@@ -45,6 +45,13 @@ def nvfp4_mm(a: NVFP4Tensor, b: NVFP4Tensor, out_dtype=None, out=None, amax_out=
                           out_dtype == torch.float32, out, amax_out)
 
 
+def mm_as(a: NVFP4Tensor, b: NVFP4Tensor, dtype) -> torch.Tensor:
+    """nvfp4_mm(a, b, torch.bfloat16).to(dtype); for fp32 the GEMM stores the rounded values itself."""
+    if dtype != torch.float32 or a._transposed or not b._transposed or a.qdata.shape[1] != b.qdata.shape[1]:
+        return nvfp4_mm(a, b, torch.bfloat16).to(dtype)
+    return _lib.host().mm_bf16_as_f32(a.qdata, a.scale, a.per_tensor_scale, b.qdata, b.scale, b.per_tensor_scale)
+
+
 def nvfp4_mm_fp4out(a: NVFP4Tensor, b: NVFP4Tensor, out_amax: torch.Tensor) -> NVFP4Tensor:
     """a @ b delivered as an NVFP4Tensor [M, N] quantized along N (round to nearest) inside the GEMM
     epilogue, for a GEMM that feeds another one: equal to quant_nvfp4(nvfp4_mm(a, b, bfloat16),

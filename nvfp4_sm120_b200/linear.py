@@ -19,7 +19,7 @@ import os
 import torch
 import torch.nn as nn
 
-from .gemm import nvfp4_mm
+from .gemm import mm_as, nvfp4_mm
 from .quant import hadamard16, quant_dual_nvfp4, quant_nvfp4, quant_weight_nvfp4, tensor_amax, tensor_amax_both
 from .tensor import BLK, NVFP4Tensor
 
@@ -160,7 +160,10 @@ class FP4LinearFn(torch.autograd.Function):
             wq_K = _quant(w, amax_reduce)
         # y_amax_out: optional fp32 [1] that the fprop GEMM's epilogue fills with max|y| (for a consumer
         # that quantizes y next; only meaningful when y stays bf16, i.e. x is bf16)
-        y = nvfp4_mm(xq, wq_K.t(), torch.bfloat16, amax_out=y_amax_out)
+        if y_amax_out is None:
+            y = mm_as(xq, wq_K.t(), x.dtype)
+        else:
+            y = nvfp4_mm(xq, wq_K.t(), torch.bfloat16, amax_out=y_amax_out).to(x.dtype)
         if xtq is None:
             ctx.save_for_backward(x2, w)
         else:
@@ -170,7 +173,7 @@ class FP4LinearFn(torch.autograd.Function):
         ctx.amax_reduce, ctx.sharded, ctx.x_amax = amax_reduce, sharded, x_amax
         ctx.x_amax_rht = bool(x_amax_rht)        # False: the Hadamard maximum came from another sign vector
         ctx.dx_reduce = dx_reduce
-        return y.reshape(*x.shape[:-1], w.shape[0]).to(x.dtype)
+        return y.reshape(*x.shape[:-1], w.shape[0])
 
     @staticmethod
     def backward(ctx, gy):
@@ -224,7 +227,7 @@ class FP4LinearFn(torch.autograd.Function):
                 gq = _quant(gy2, None if g_amax is not None else g_red, stochastic=True, amax=g_amax, counter=ctr_rows)
             if wq_N is None:
                 wq_N = _quant(w, red, transpose=True)
-            dx = nvfp4_mm(gq, wq_N.t(), torch.bfloat16).reshape(ctx.xshape).to(gy.dtype)
+            dx = mm_as(gq, wq_N.t(), gy.dtype).reshape(ctx.xshape)
         pending = ctx.dx_reduce(dx) if (dx is not None and ctx.dx_reduce is not None) else None
         if ctx.needs_input_grad[1]:
             # wgrad: dW = dY^T @ X, contraction over tokens; Hadamard on both, SR on the gradient
