@@ -87,10 +87,10 @@ def _take_grad_amax(gy2, signs=None):
 
 
 _DUAL = [True]
-# The one-read kernel wins where launches and re-reads dominate (measured on a B200: 43 us against 64 us
-# for the two layouts of a 4096 x 4096 tensor) and loses to the two streaming kernels on large tensors
-# (150 us against 127 us at 4096 x 28672), so it takes tensors up to this many elements.
-_DUAL_MAX_ELEMS = 1 << 24
+# The one-read kernel wins wherever a second read, launch or maximum counts (measured on a B200, maxima given, us, one
+# kernel against two: 16384 x 768 nearest 15.9 / 19.3, stochastic 21.3 / 24.9; 4096 x 14336 53 / 62 and 76 / 78) and is
+# level with the two at 4096 x 28672 stochastic (144 / 143), so it takes tensors up to this many elements.
+_DUAL_MAX_ELEMS = 1 << 26
 
 
 def set_dual_quant(flag: bool):
@@ -117,7 +117,7 @@ class FP4LinearFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w, H, signs, wq_K, wq_N, amax_reduce=None, sharded=(False, False), x_amax=None,
-                x_amax_rht=True, dx_reduce=None, y_amax_out=None, x_quant=None):
+                x_amax_rht=True, dx_reduce=None, y_amax_out=None, x_quant=None, grad_on=False):
         # dx_reduce: optional callable(dx) -> handle with .wait(): starts the sum of the input gradient
         # over a tensor-parallel group right after the dgrad GEMM, so that it runs beside the wgrad
         # quantizations and GEMM; the handle is waited for before the backward returns
@@ -142,8 +142,9 @@ class FP4LinearFn(torch.autograd.Function):
         # x nor another pass in backward.  (A sharded x without producer maxima keeps the two-step path:
         # its maxima are reduced over the group one by one.)
         have_both = x_amax is not None and x_amax_rht and x_amax.numel() >= 2
-        # (inside torch.no_grad() needs_input_grad still reflects requires_grad: ask the grad mode too)
-        dual = (_DUAL[0] and ctx.needs_input_grad[1] and torch.is_grad_enabled() and x2.is_cuda and x2.shape[0] % BLK == 0
+        # grad_on: is a backward to come?  The caller says so: inside torch.no_grad() needs_input_grad still reflects
+        # requires_grad, and the grad mode is always off in here.
+        dual = (_DUAL[0] and ctx.needs_input_grad[1] and grad_on and x2.is_cuda and x2.shape[0] % BLK == 0
                 and x2.numel() <= _DUAL_MAX_ELEMS and (x_red is None) and (have_both or not x_sharded))
         xtq = None
         if x_quant is not None:
@@ -239,7 +240,7 @@ class FP4LinearFn(torch.autograd.Function):
             dw = nvfp4_mm(gtq, xtq.t(), _grad_dtype(w)).to(w.dtype)
         if pending is not None:
             pending.wait()
-        return dx, dw, None, None, None, None, None, None, None, None, None, None, None
+        return dx, dw, None, None, None, None, None, None, None, None, None, None, None, None
 
 
 def _quant(t, amax_reduce, stochastic=False, rht=False, H=None, signs=None, transpose=False, amax=None, counter=None):
@@ -332,9 +333,13 @@ class FP4Linear(nn.Module):
         if x.is_cuda and torch.is_autocast_enabled("cuda"):
             x = x.to(torch.get_autocast_dtype("cuda"))       # what autocast does for nn.Linear
         wq_K, wq_N = self._cache.get(self.weight)
+        grad_on = torch.is_grad_enabled()
+        if wq_K is None and grad_on and x.requires_grad:
+            # both layouts of the weight from one read: fprop's operand now, dgrad's for the backward
+            wq_K, wq_N = quant_weight_nvfp4(self.weight.detach())
         rht_ok = amax_signs is None or _same_signs(amax_signs, self.signs)
         return FP4LinearFn.apply(x, self.weight, self.H, self.signs, wq_K, wq_N, None, (False, False), amax, rht_ok,
-                                 None, amax_out, x_quant)
+                                 None, amax_out, x_quant, grad_on)
 
     def extra_repr(self):
         return f"in_features={self.weight.shape[1]}, out_features={self.weight.shape[0]}, bias=False, nvfp4"
