@@ -204,10 +204,12 @@ class FP4LinearFn(torch.autograd.Function):
                   and gy2.shape[0] % BLK == 0 and gy2.numel() <= _DUAL_MAX_ELEMS
                   and (g_red is None or ctr_rows is not None))
         if dual_g and (g_amax is None or g_amax_rht is None):
-            both = tensor_amax_both(gy2, signs)               # one read for the two maxima
             if g_red is not None:
+                both = tensor_amax_both(gy2, signs)           # one read for the two maxima
                 g_red(both)
-            g_amax, g_amax_rht = both[0:1], both[1:2]
+                g_amax, g_amax_rht = both[0:1], both[1:2]
+            else:                                             # the quantization below finds them, with the rounding of
+                g_amax = g_amax_rht = None                    # an fp32 gradient in the same read
         elif g_amax is not None and g_red is not None:
             # a sharded gradient: reduce the producer's maxima over the group, both in ONE collective
             both = torch.cat([g_amax, g_amax_rht]) if g_amax_rht is not None else g_amax.clone()
