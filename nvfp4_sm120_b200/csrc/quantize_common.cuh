@@ -99,6 +99,16 @@ __device__ __forceinline__ void mul2_poszero(float a, float b, float s, float& d
       " fma.rn.f32x2 r, p, q, z; mov.b64 {%0, %1}, r;}"
       : "=f"(d0), "=f"(d1) : "f"(a), "f"(b), "f"(s), "f"(0.0f));
 }
+// (a, b) * (s, t) + (0, 0): mul2_poszero with a factor for each lane
+__device__ __forceinline__ void mul2_pair_poszero(float a, float b, float s, float t, float& d0, float& d1) {
+  asm("{.reg .b64 p, q, r, z; mov.b64 p, {%2, %3}; mov.b64 q, {%4, %5}; mov.b64 z, {%6, %6};"
+      " fma.rn.f32x2 r, p, q, z; mov.b64 {%0, %1}, r;}"
+      : "=f"(d0), "=f"(d1) : "f"(a), "f"(b), "f"(s), "f"(t), "f"(0.0f));
+}
+__device__ __forceinline__ void mul2_pair(float a, float b, float s, float t, float& d0, float& d1) {
+  asm("{.reg .b64 p, q, r; mov.b64 p, {%2, %3}; mov.b64 q, {%4, %5}; mul.rn.f32x2 r, p, q; mov.b64 {%0, %1}, r;}"
+      : "=f"(d0), "=f"(d1) : "f"(a), "f"(b), "f"(s), "f"(t));
+}
 // (a0, a1) and (b0, b1) -> sums into a, differences into b
 __device__ __forceinline__ void addsub2(float& a0, float& a1, float& b0, float& b1) {
   float s0, s1, d0, d1;

@@ -74,20 +74,10 @@ __device__ __forceinline__ fused::Scale global_scale(float amax) {
   return s;
 }
 
-// v[16] -> codes and scale byte, the arithmetic of every quantizer here (quantize_common.cuh).
-// POSZERO: an exact zero that left the butterfly as -0 becomes +0
-template <bool SR, bool POSZERO>
-__device__ __forceinline__ void encode(const float (&v)[16], float amax_b, const fused::Scale& sc, const float* recip_tab,
-                                       uint64_t counter, const PhiloxKeys& keys, uint64_t offset, uint32_t& lo,
-                                       uint32_t& hi, uint32_t& sf) {
-  sf = fused::block_scale_byte(amax_b, sc);
-  const float recip = recip_tab[sf];
-  float d[16];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    if (POSZERO) fused::mul2_poszero(v[2 * j], v[2 * j + 1], recip, d[2 * j], d[2 * j + 1]);
-    else fused::mul2(v[2 * j], v[2 * j + 1], recip, d[2 * j], d[2 * j + 1]);
-  }
+// d[16] = the scaled values of a block -> codes
+template <bool SR>
+__device__ __forceinline__ void encode(const float (&d)[16], uint64_t counter, const PhiloxKeys& keys, uint64_t offset,
+                                       uint32_t& lo, uint32_t& hi) {
   if (SR) {
     const Philox4 r = fused::philox_rounds((uint32_t)counter, (uint32_t)(counter >> 32), (uint32_t)offset,
                                            (uint32_t)(offset >> 32), keys);
@@ -172,7 +162,8 @@ quant_dual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     // ---- transposed: this warp's half and 16-row block, two columns per lane
     if (do_cols) {
       const uint32_t half = warp & 1u, rb = warp >> 1;
-      const uint32_t addr = fused::smem_u32(slot) + half * kHalfBytes + rb * 2048u + (lane & 3u) * 4u;
+      // 128-byte swizzle: 16-byte chunk c of row k sits at c ^ (k & 7)
+      const uint32_t addr = fused::smem_u32(slot) + half * kHalfBytes + rb * 2048u + lane * 4u;
       float v0[16], v1[16];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -183,7 +174,7 @@ quant_dual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         for (int e = 0; e < 4; ++e) {
           const int k = 4 * q + e;
           uint32_t w;
-          asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"((addr + (((lane >> 2) ^ (k & 7)) << 4)) + 128 * k));
+          asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"((addr ^ ((uint32_t)(k & 7) << 4)) + 128 * k));
           v0[k] = __uint_as_float((w << 16) + m[e]);                     // adding the top bit flips the sign: one
           v1[k] = __uint_as_float((w & 0xffff0000u) ^ m[e]);             // instruction each with the unpacking
         }
@@ -203,15 +194,23 @@ quant_dual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       const int64_t kb = (r0 >> 4) + rb;
       const uint32_t c = half * 64u + 2u * lane;                         // column inside the tile
       const uint64_t ctr = (uint64_t)(c0 + c) * p.pitch_c + p.base_c + (uint64_t)kb;
+      // both columns' values stay paired up to the conversion
+      const uint32_t sf0 = fused::block_scale_byte(fused::max_abs16(v0) * rht_scale, sc_c);
+      const uint32_t sf1 = fused::block_scale_byte(fused::max_abs16(v1) * rht_scale, sc_c);
+      const float rc0 = recip_c[sf0], rc1 = recip_c[sf1];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {                                     // an exact zero that left the butterfly as -0: +0
+        if (RHT) fused::mul2_pair_poszero(v0[k], v1[k], rc0, rc1, v0[k], v1[k]);
+        else fused::mul2_pair(v0[k], v1[k], rc0, rc1, v0[k], v1[k]);
+      }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const float(&v)[16] = h ? v1 : v0;
-        uint32_t lo, hi, sf;
-        encode<SR_C, RHT>(v, fused::max_abs16(v) * rht_scale, sc_c, recip_c, ctr + (h ? p.pitch_c : 0ull), p.keys_c,
-                          p.offset, lo, hi, sf);
+        uint32_t lo, hi;
+        encode<SR_C>(h ? v1 : v0, ctr + (h ? p.pitch_c : 0ull), p.keys_c, p.offset, lo, hi);
         *reinterpret_cast<uint2*>(out + (c + h) * kOutPitch + rb * 8u) = make_uint2(lo, hi);
         const bool inside = c0 + c + h < p.cols && kb < blk_c;
-        out_sf[(rb >> 2) * 512u + ((c + h) & 31u) * 16u + ((c + h) >> 5) * 4u + (rb & 3u)] = inside ? (uint8_t)sf : (uint8_t)0;
+        out_sf[(rb >> 2) * 512u + ((c + h) & 31u) * 16u + ((c + h) >> 5) * 4u + (rb & 3u)] =
+            inside ? (uint8_t)(h ? sf1 : sf0) : (uint8_t)0;
       }
     }
     // ---- row-wise: blocks (row_t, kb) of the two halves
@@ -231,9 +230,12 @@ quant_dual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         float v[16];
 #pragma unroll
         for (int j = 0; j < 8; ++j) { v[2 * j] = bf16_lo(w[j]); v[2 * j + 1] = bf16_hi(w[j]); }
-        uint32_t lo, hi, sf;
-        encode<ROWS == 2, false>(v, fused::amax_packed8(w), sc_r, recip_r,
-                                 (uint64_t)r * p.pitch_r + p.base_r + (uint64_t)kb, p.keys_r, p.offset, lo, hi, sf);
+        uint32_t lo, hi;
+        const uint32_t sf = fused::block_scale_byte(fused::amax_packed8(w), sc_r);
+        const float recip = recip_r[sf];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) fused::mul2(v[2 * j], v[2 * j + 1], recip, v[2 * j], v[2 * j + 1]);
+        encode<ROWS == 2>(v, (uint64_t)r * p.pitch_r + p.base_r + (uint64_t)kb, p.keys_r, p.offset, lo, hi);
         const bool inside = r < p.rows && kb < blk_r;
         if (inside) *reinterpret_cast<uint2*>(p.q_r + r * (p.cols >> 1) + kb * 8) = make_uint2(lo, hi);
         p.sf_r[((r0 >> 7) * ct_r + (c0 >> 6) + half) * 512 + (2u * warp + hrow) * 16u + grp * 4u + kb4] =
