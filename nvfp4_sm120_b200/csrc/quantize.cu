@@ -274,12 +274,6 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const uint16_t* __restr
   }
 }
 
-// ---------------------------------------------------------------------------------------
-// transposing variants: blocks along the ROWS of x; the output describes x^T [cols, rows].
-// A thread owns two adjacent columns and up to 64 consecutive rows (four 16-row blocks), so
-// that a warp reads 128 contiguous bytes per row and each thread writes 32 contiguous output
-// bytes per column.
-// ---------------------------------------------------------------------------------------
 // The 16-point butterfly of two adjacent columns at once: (v0[i], v1[i]) ride in the two lanes of the
 // packed fp32 add / sub / fma, half the instructions of two scalar butterflies and the same bits
 // (same operations in the same order as hadamard16_inplace, exact zeros made +0).
@@ -301,58 +295,12 @@ __device__ __forceinline__ void sign_masks(const float (&sg)[16], uint32_t (&sm)
   for (int i = 0; i < 16; ++i) sm[i] = sg[i] < 0.0f ? 0x80008000u : 0u;
 }
 
-template <bool RHT>
-__device__ __forceinline__ void load_col_pair_block(const uint16_t* __restrict__ x, int64_t ld,
-                                                    int64_t r0, int64_t c, const uint32_t (&sm)[16],
-                                                    float (&v0)[16], float (&v1)[16]) {
-  const uint32_t* p = reinterpret_cast<const uint32_t*>(x + r0 * ld + c);
-  uint32_t w[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) w[i] = __ldg(p + (size_t)i * (size_t)(ld >> 1));
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const uint32_t u = RHT ? (w[i] ^ sm[i]) : w[i];      // times +-1 = a flip of the sign bit
-    v0[i] = bf16_lo(u);
-    v1[i] = bf16_hi(u);
-  }
-  if (RHT) hadamard16_pair(v0, v1);
-}
-
-__global__ void __launch_bounds__(256) amax_rht_cols_kernel(const uint16_t* __restrict__ x, int64_t rows,
-                                                            int64_t cols, int64_t ld,
-                                                            const float* __restrict__ signs16,
-                                                            float* __restrict__ amax) {
-  float sg[16];
-  load_signs(signs16, sg);
-  uint32_t sm[16];
-  sign_masks(sg, sm);
-  const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
-  const int64_t r_base = (int64_t)blockIdx.y * 64;
-  float m = 0.0f;
-  if (c < cols) {
-#pragma unroll 1
-    for (int j = 0; j < 4; ++j) {
-      const int64_t r0 = r_base + 16 * j;
-      if (r0 >= rows) break;
-      float v0[16], v1[16];
-      load_col_pair_block<true>(x, ld, r0, c, sm, v0, v1);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) m = fmaxf(m, fmaxf(fabsf(v0[i]), fabsf(v1[i])));
-    }
-  }
-  cta_max_to(amax, m);
-}
-
 // ---------------------------------------------------------------------------------------
-// Wide form of the column MAXIMUM kernels for 16-byte rows (cols % 8 == 0).  The narrow kernels above read
-// 128 contiguous bytes of a row per warp instruction; here a CTA takes tiles of 16 rows x 512 columns
-// the way the activation kernels do (csrc/swiglu.cu): thread t and step k load the eight columns
-// 8 * (t % 64) of row 4k + t / 64 with one 16-byte load (a warp moves 512 contiguous bytes of a row),
-// the tile goes to padded shared memory, and thread t then reads its two columns of all 16 rows from
-// there (consecutive lanes, consecutive banks), with the next tile's loads in flight.  Measured on a
-// B200 at 4096 x 4096: both maxima 14.9 us against 17.1 us.  The same staging for the quantizer itself
-// was slower (116 us against 89.5 us at 4096 x 28672, RHT + stochastic): its long encode phase leaves
-// only the four prefetch loads per thread in flight, so quant_cols_kernel keeps its direct loads.
+// Both maxima of an fp32 matrix's bf16 rounding, which goes to memory on the way (16-byte rows, cols % 8 == 0).  A CTA
+// takes tiles of 16 rows x 512 columns the way the activation kernels do (csrc/swiglu.cu): thread t and step k load the
+// eight columns 8 * (t % 64) of row 4k + t / 64, the rounded tile goes to padded shared memory, and thread t then
+// reads its two columns of all 16 rows from there (consecutive lanes, consecutive banks), with the next tile's loads in
+// flight.  bf16 matrices: quantize_dual.cu.
 // ---------------------------------------------------------------------------------------
 constexpr int kWideCols = 512;
 constexpr int kWidePitch = kWideCols / 2 + 4;            // 32-bit words per tile row, padded
@@ -372,15 +320,6 @@ __device__ __forceinline__ WideTile wide_tile(int64_t cols) {
   t.c = t.c0 + 2 * (int64_t)threadIdx.x;
   t.mine = t.c < cols;
   return t;
-}
-__device__ __forceinline__ void wide_fetch(const uint16_t* __restrict__ x, int64_t rows, int64_t ld, const WideTile& t,
-                                           int j, uint4 (&d)[4]) {
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int64_t r = t.r_base + 16 * j + 4 * k + t.lr;
-    d[k] = (t.col_in && r < rows) ? __ldg(reinterpret_cast<const uint4*>(x + r * ld + t.c0 + t.cc))
-                                  : make_uint4(0u, 0u, 0u, 0u);
-  }
 }
 __device__ __forceinline__ void wide_stage(uint32_t* tile, const WideTile& t, const uint4 (&d)[4]) {
 #pragma unroll
@@ -407,16 +346,10 @@ __device__ __forceinline__ void wide_fetch_round(const float* __restrict__ x, in
   }
 }
 
-// BOTH: maxima2[0] = plain maximum as well (else only maxima2[0] = maximum after the transform).  F32: x is fp32, the
-// maxima are those of its bf16 rounding, which goes to `rounded`.
-template <bool BOTH, bool F32>
-__global__ void __launch_bounds__(256) amax_cols_wide_kernel(const void* __restrict__ x, int64_t rows, int64_t cols,
-                                                             int64_t ld, const float* __restrict__ signs16,
-                                                             float* __restrict__ out, uint16_t* __restrict__ rounded) {
-  auto fetch = [&](const WideTile& t, int j, uint4 (&d)[4]) {
-    if (F32) wide_fetch_round(static_cast<const float*>(x), rows, cols, ld, t, j, rounded, d);
-    else wide_fetch(static_cast<const uint16_t*>(x), rows, ld, t, j, d);
-  };
+// out[0] = plain maximum, out[1] = maximum after the transform
+__global__ void __launch_bounds__(256) round_amax_both_kernel(const float* __restrict__ x, int64_t rows, int64_t cols,
+                                                              int64_t ld, const float* __restrict__ signs16,
+                                                              float* __restrict__ out, uint16_t* __restrict__ rounded) {
   __shared__ __align__(16) uint32_t tile[16 * kWidePitch];
   float sg[16];
   load_signs(signs16, sg);
@@ -426,20 +359,18 @@ __global__ void __launch_bounds__(256) amax_cols_wide_kernel(const void* __restr
   float m = 0.0f;
   uint32_t mp = 0u;
   uint4 nxt[4];
-  fetch(t, 0, nxt);
+  wide_fetch_round(x, rows, cols, ld, t, 0, rounded, nxt);
 #pragma unroll 1
   for (int j = 0; j < 4; ++j) {
     if (t.r_base + 16 * j >= rows) break;                  // uniform over the CTA
     wide_stage(tile, t, nxt);
-    if (BOTH) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t kk = 0x7fff7fffu;
-        mp = __vimax3_u16x2(mp, nxt[k].x & kk, nxt[k].y & kk);
-        mp = __vimax3_u16x2(mp, nxt[k].z & kk, nxt[k].w & kk);
-      }
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t kk = 0x7fff7fffu;
+      mp = __vimax3_u16x2(mp, nxt[k].x & kk, nxt[k].y & kk);
+      mp = __vimax3_u16x2(mp, nxt[k].z & kk, nxt[k].w & kk);
     }
-    if (j + 1 < 4) fetch(t, j + 1, nxt);
+    if (j + 1 < 4) wide_fetch_round(x, rows, cols, ld, t, j + 1, rounded, nxt);
     __syncthreads();
     if (t.mine) {
       float v0[16], v1[16];
@@ -455,13 +386,9 @@ __global__ void __launch_bounds__(256) amax_cols_wide_kernel(const void* __restr
     }
     __syncthreads();
   }
-  if (BOTH) {
-    mp = max(mp & 0xffffu, mp >> 16);
-    cta_max_to(out, __uint_as_float(mp << 16), 0);
-    cta_max_to(out + 1, m, 1);
-  } else {
-    cta_max_to(out, m);
-  }
+  mp = max(mp & 0xffffu, mp >> 16);
+  cta_max_to(out, __uint_as_float(mp << 16), 0);
+  cta_max_to(out + 1, m, 1);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -537,44 +464,6 @@ __global__ void __launch_bounds__(256) quant_weight_2d_kernel(const uint16_t* __
 }
 
 
-// plain maximum and maximum after the Hadamard transform along the rows, from one read
-__global__ void __launch_bounds__(256) amax_both_cols_kernel(const uint16_t* __restrict__ x, int64_t rows,
-                                                             int64_t cols, int64_t ld,
-                                                             const float* __restrict__ signs16,
-                                                             float* __restrict__ maxima2) {
-  float sg[16];
-  load_signs(signs16, sg);
-  uint32_t sm[16];
-  sign_masks(sg, sm);
-  const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
-  const int64_t r_base = (int64_t)blockIdx.y * 64;
-  float m = 0.0f;
-  uint32_t mp = 0u;
-  if (c < cols) {
-#pragma unroll 1
-    for (int j = 0; j < 4; ++j) {
-      const int64_t r0 = r_base + 16 * j;
-      if (r0 >= rows) break;
-      const uint32_t* p = reinterpret_cast<const uint32_t*>(x + r0 * ld + c);
-      float v0[16], v1[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const uint32_t w = __ldg(p + (size_t)i * (size_t)(ld >> 1));
-        mp = __vimax3_u16x2(mp, w & 0x7fff7fffu, 0u);          // both halves carry a running maximum
-        const uint32_t u = w ^ sm[i];
-        v0[i] = bf16_lo(u);
-        v1[i] = bf16_hi(u);
-      }
-      hadamard16_pair(v0, v1);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) m = fmaxf(m, fmaxf(fabsf(v0[i]), fabsf(v1[i])));
-    }
-  }
-  mp = max(mp & 0xffffu, mp >> 16);
-  cta_max_to(maxima2, __uint_as_float(mp << 16), 0);
-  cta_max_to(maxima2 + 1, m, 1);
-}
-
 static inline int grid_for(int64_t work_items, int threads, int max_blocks) {
   int64_t b = (work_items + threads - 1) / threads;
   if (b > max_blocks) b = max_blocks;
@@ -588,6 +477,14 @@ using namespace nvfp4;
 
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+namespace nvfp4 { namespace dual {
+int launch_amax(const void* x, int64_t rows, int64_t cols, int64_t ld, const float* signs16, bool both, float* out,
+                cudaStream_t stream);
+int launch(const void* x, int64_t rows, int64_t cols, int64_t ld, int rows_mode, bool sr_c, const float* signs16,
+           const float* amax_r, const float* amax_c, uint64_t seed_r, uint64_t seed_c, uint64_t offset,
+           const uint64_t* counters4, uint8_t* q_r, uint8_t* sf_r, float* pts_r, uint8_t* q_c, uint8_t* sf_c, float* pts_c,
+           cudaStream_t stream);
+}}
 extern "C" int nvfp4_amax_bf16(const void* x, int64_t rows, int64_t cols, int64_t ld, int rht,
                                int transpose, const float* signs16, float* amax, int zero_first,
                                void* stream_) {
@@ -607,24 +504,12 @@ extern "C" int nvfp4_amax_bf16(const void* x, int64_t rows, int64_t cols, int64_
     amax_rht_rows_kernel<<<grid_for(rows * bpr, 256 * 2, 148 * 16), 256, 0, stream>>>(xp, rows, bpr, ld, signs16, amax);
   } else {
     if ((rows & 15) != 0 || (cols & 1) != 0) return NVFP4_E_SHAPE;
-    dim3 grid((unsigned)((cols / 2 + 255) / 256), (unsigned)((rows + 63) / 64));
-    if (grid.y > 65535u) return NVFP4_E_SHAPE;
-    if ((cols & 7) == 0) {
-      const dim3 wgrid((unsigned)((cols + kWideCols - 1) / kWideCols), grid.y);
-      amax_cols_wide_kernel<false, false><<<wgrid, 256, 0, stream>>>(xp, rows, cols, ld, signs16, amax, nullptr);
-    } else {
-      amax_rht_cols_kernel<<<grid, 256, 0, stream>>>(xp, rows, cols, ld, signs16, amax);
-    }
+    if ((rows + 63) / 64 > 65535) return NVFP4_E_SHAPE;
+    return nvfp4::dual::launch_amax(x, rows, cols, ld, signs16, false, amax, stream);
   }
   return cudaGetLastError() == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
 }
 
-namespace nvfp4 { namespace dual {
-int launch(const void* x, int64_t rows, int64_t cols, int64_t ld, int rows_mode, bool sr_c, const float* signs16,
-           const float* amax_r, const float* amax_c, uint64_t seed_r, uint64_t seed_c, uint64_t offset,
-           const uint64_t* counters4, uint8_t* q_r, uint8_t* sf_r, float* pts_r, uint8_t* q_c, uint8_t* sf_c, float* pts_c,
-           cudaStream_t stream);
-}}
 namespace nvfp4 { namespace fused {
 int quantize_rows_known_amax(const void* x, int64_t rows, int64_t cols, int64_t ld, int mode, int rht,
                              const float* signs16, const float* amax, uint64_t seed, uint64_t offset,
@@ -714,15 +599,8 @@ extern "C" int nvfp4_amax_both_bf16(const void* x, int64_t rows, int64_t cols, i
   if (rows <= 0 || cols <= 0 || ld < cols || (rows & 15) != 0 || (cols & 1) != 0) return NVFP4_E_SHAPE;
   if (!aligned16(x) || (ld & 7) != 0 || !aligned16(signs16)) return NVFP4_E_ALIGN;
   if (zero_first && cudaMemsetAsync(maxima2, 0, 2 * sizeof(float), stream) != cudaSuccess) return NVFP4_E_LAUNCH;
-  dim3 grid((unsigned)((cols / 2 + 255) / 256), (unsigned)((rows + 63) / 64));
-  if (grid.y > 65535u) return NVFP4_E_LIMIT;
-  if ((cols & 7) == 0) {
-    const dim3 wgrid((unsigned)((cols + kWideCols - 1) / kWideCols), grid.y);
-    amax_cols_wide_kernel<true, false><<<wgrid, 256, 0, stream>>>(x, rows, cols, ld, signs16, maxima2, nullptr);
-  } else {
-    amax_both_cols_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(x), rows, cols, ld, signs16, maxima2);
-  }
-  return cudaGetLastError() == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
+  if ((rows + 63) / 64 > 65535) return NVFP4_E_LIMIT;
+  return nvfp4::dual::launch_amax(x, rows, cols, ld, signs16, true, maxima2, stream);
 }
 
 extern "C" int nvfp4_round_amax_f32(const float* x, int64_t rows, int64_t cols, int64_t ld, void* out_bf16,
@@ -738,7 +616,7 @@ extern "C" int nvfp4_round_amax_f32(const float* x, int64_t rows, int64_t cols, 
   uint16_t* out = static_cast<uint16_t*>(out_bf16);
   if (signs16 != nullptr) {
     const dim3 grid((unsigned)((cols + kWideCols - 1) / kWideCols), (unsigned)((rows + 63) / 64));
-    amax_cols_wide_kernel<true, true><<<grid, 256, 0, stream>>>(x, rows, cols, ld, signs16, maxima, out);
+    round_amax_both_kernel<<<grid, 256, 0, stream>>>(x, rows, cols, ld, signs16, maxima, out);
   } else {
     const int vpr = (int)(cols >> 3);
     round_amax_kernel<<<grid_for(rows * vpr, 512 * 2, 148 * 4), 512, 0, stream>>>(x, rows, vpr, ld, out, maxima);

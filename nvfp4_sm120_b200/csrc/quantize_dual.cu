@@ -17,10 +17,10 @@
 // on the half-rate ALU pipe), not memory.
 // Measured, maxima given, HBM-cold, us (before = one 64 x 64 tile per 256-thread CTA, and for the transposed output alone
 // two columns x 64 rows per thread straight from global memory):
-//   4096 x 28672   transposed nearest 68.2 -> 49.8, RHT 74.6 -> 61.1, RHT + stochastic 87.9 -> 85.7; both layouts
-//                  nearest 169.6 -> 98.4, stochastic 192.5 -> 143.9; a weight in both layouts 123.7 -> 83.6
-//   16384 x 768    transposed RHT + stochastic 17.2 -> 14.1, both layouts stochastic 24.4 -> 21.3
-//   512 x 768      transposed RHT + stochastic 6.6 -> 4.3, both layouts stochastic 4.0 -> 4.7, a weight 3.1 -> 3.8
+//   4096 x 28672   transposed nearest 68.2 -> 49.8, RHT 74.6 -> 61.1, RHT + stochastic 87.9 -> 80; both layouts
+//                  nearest 169.6 -> 98.4, stochastic 192.5 -> 139; a weight in both layouts 123.7 -> 83.6
+//   16384 x 768    transposed RHT + stochastic 17.2 -> 13.5, both layouts stochastic 24.4 -> 20.9
+//   512 x 768      transposed RHT + stochastic 6.6 -> 4.0, both layouts stochastic 4.0 -> 4.4, a weight 3.1 -> 3.7
 // Rows and columns outside the matrix get zero scale bytes, so the padding of the scale buffers needs no clearing.
 #include <mutex>
 
@@ -270,6 +270,112 @@ quant_dual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// The maxima of the same tiles: after the Hadamard transform along the rows, and with BOTH the plain one too
+// (out[0] = plain, out[1] = transformed; without BOTH out[0] = transformed).  Three slots of 32 KiB per CTA, two CTAs per
+// SM: 192 KiB in flight or in work per SM, one atomic per CTA and maximum.  HBM-bound, us with the clearing of the words,
+// both maxima: 4096 x 28672 51.5 -> 42.0 (5.6 TB/s), 4096 x 14336 30.8 -> 25.1, 4096 x 4096 14.7 -> 12.7, 16384 x 768
+// 14.7 -> 11.4, 512 x 768 7.3 -> 6.4 (before: a CTA per 64 rows x 512 columns, staged through registers, thousands of CTAs).
+// ---------------------------------------------------------------------------------------
+constexpr int kMaxSlots = 3;
+constexpr int kMaxMiscOff = kMaxSlots * kSlotBytes;
+constexpr int kMaxSmemBytes = kMaxMiscOff + 512 /* signs, barriers, partial maxima */ + 1024 /* alignment slack */;
+
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
+template <bool BOTH>
+__global__ void __launch_bounds__(kThreads, 2)
+amax_tiles_kernel(const __grid_constant__ CUtensorMap map_x, uint32_t ntc, uint32_t ntiles,
+                  const float* __restrict__ signs16, float* __restrict__ out) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = fused::smem_u32(smem_raw);
+  uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
+  uint32_t* sgn = reinterpret_cast<uint32_t*>(smem + kMaxMiscOff);       // 16 sign-flip masks
+  float* part = reinterpret_cast<float*>(sgn + 16);                       // 2 x 16 warp maxima
+  const uint32_t bars = fused::smem_u32(part + 32);
+  volatile int* gave_up = reinterpret_cast<volatile int*>(part + 32 + 2 * kMaxSlots);
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t my_tiles = blockIdx.x < ntiles ? (ntiles - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
+  auto fetch = [&](uint32_t i) {
+    const uint32_t tile = blockIdx.x + i * gridDim.x, rt = tile / ntc, ct = tile - rt * ntc;
+    const uint32_t s = i % kMaxSlots, bar = bars + 8u * s, dst = fused::smem_u32(smem) + s * kSlotBytes;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)kSlotBytes) : "memory");
+    tma_half_load(dst, &map_x, (int)(ct * kTile), (int)(rt * kTile), bar);
+    tma_half_load(dst + kHalfBytes, &map_x, (int)(ct * kTile + 64), (int)(rt * kTile), bar);
+  };
+  if (tid == 0) {
+    for (int s = 0; s < kMaxSlots; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8u * s));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    *gave_up = 0;
+    for (uint32_t i = 0; i < (uint32_t)kMaxSlots && i < my_tiles; ++i) fetch(i);
+  }
+  if (tid >= 32 && tid < 48) sgn[tid - 32] = __ldg(signs16 + (tid - 32)) < 0.0f ? 0x80000000u : 0u;
+  __syncthreads();
+  float m = 0.0f;
+  uint32_t mp = 0u;                                // both 16-bit halves carry a running maximum of bf16 magnitudes
+  const uint32_t half = warp & 1u, rb = warp >> 1;
+  for (uint32_t i = 0; i < my_tiles; ++i) {
+    const uint32_t slot = (i % kMaxSlots) * kSlotBytes, bar = bars + 8u * (i % kMaxSlots), parity = (i / kMaxSlots) & 1u;
+    if (!fused::mbar_try_wait(bar, parity)) {
+      const unsigned long long t0 = fused::global_ns();
+      while (!fused::mbar_try_wait(bar, parity)) {
+        if (fused::global_ns() - t0 > fused::kWaitLimitNs) { *gave_up = 1; break; }
+      }
+    }
+    const uint32_t addr = fused::smem_u32(smem) + slot + half * kHalfBytes + rb * 2048u + lane * 4u;
+    float v0[16], v1[16];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint4 m4 = reinterpret_cast<const uint4*>(sgn)[q];
+      const uint32_t sm[4] = {m4.x, m4.y, m4.z, m4.w};
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int k = 4 * q + e;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[e]) : "r"((addr ^ ((uint32_t)(k & 7) << 4)) + 128 * k));
+        v0[k] = __uint_as_float((w[e] << 16) + sm[e]);
+        v1[k] = __uint_as_float((w[e] & 0xffff0000u) ^ sm[e]);
+      }
+      if (BOTH) {
+        const uint32_t kk = 0x7fff7fffu;
+        mp = __vimax3_u16x2(__vimax3_u16x2(mp, w[0] & kk, w[1] & kk), w[2] & kk, w[3] & kk);
+      }
+    }
+#pragma unroll
+    for (int s = 1; s < 16; s <<= 1) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        if ((k & s) == 0) fused::addsub2(v0[k], v1[k], v0[k | s], v1[k | s]);
+    }
+    m = fmaxf(m, fmaxf(fused::max_abs16(v0), fused::max_abs16(v1)));
+    __syncthreads();                                                      // the slot is read
+    if (*gave_up != 0) break;
+    if (tid == 0 && i + kMaxSlots < my_tiles) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");        // generic reads before the async write
+      fetch(i + kMaxSlots);
+    }
+  }
+  const float plain = __uint_as_float(max(mp & 0xffffu, mp >> 16) << 16);
+  // a NaN has the largest bit pattern: the plain maximum compares bits, as the plain kernel's does
+  const uint32_t plain_bits = __reduce_max_sync(0xffffffffu, __float_as_uint(plain));
+  m = warp_max(m * 0.25f);                                                // the transform is butterfly / 4
+  if (lane == 0) { part[warp] = m; part[16 + warp] = __uint_as_float(plain_bits); }
+  __syncthreads();
+  if (warp == 0) {
+    const float r = warp_max(lane < 16 ? part[lane] : 0.0f);
+    const uint32_t pb = __reduce_max_sync(0xffffffffu, lane < 16 ? __float_as_uint(part[16 + lane]) : 0u);
+    if (lane == 0) {
+      unsigned int* o = reinterpret_cast<unsigned int*>(out);             // non-negative floats order like their bits
+      if (BOTH && pb != 0u) atomicMax(o, pb);
+      if (r > 0.0f) atomicMax(o + (BOTH ? 1 : 0), __float_as_uint(r));
+    }
+  }
+}
+
 namespace {
 std::mutex g_mutex;
 int g_sms[64];
@@ -295,6 +401,11 @@ int sm_count(int& out) {
         cudaGetLastError();
         return NVFP4_E_LAUNCH;
       }
+    if (cudaFuncSetAttribute(amax_tiles_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes) != cudaSuccess ||
+        cudaFuncSetAttribute(amax_tiles_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes) != cudaSuccess) {
+      cudaGetLastError();
+      return NVFP4_E_LAUNCH;
+    }
     g_sms[dev] = sms;
   }
   out = g_sms[dev];
@@ -311,6 +422,35 @@ static PhiloxKeys make_keys(uint64_t seed) {
   return keys;
 }
 
+// tiles of 128 rows x 64 columns of x [rows, cols] bf16, row pitch ld
+static bool make_tile_map(CUtensorMap* map, const void* x, int64_t rows, int64_t cols, int64_t ld) {
+  gemm::EncodeTiledFn enc = gemm::encode_fn();
+  if (enc == nullptr) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 2u};
+  cuuint32_t box[2] = {64u, (cuuint32_t)kTile};
+  cuuint32_t estr[2] = {1u, 1u};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The maxima of x, into words that are zero: the transformed one, or (both) the plain one and the transformed one.
+int launch_amax(const void* x, int64_t rows, int64_t cols, int64_t ld, const float* signs16, bool both, float* out,
+                cudaStream_t stream) {
+  int sms = 0;
+  const int rc = sm_count(sms);
+  if (rc != NVFP4_OK) return rc;
+  CUtensorMap map;
+  if (!make_tile_map(&map, x, rows, cols, ld)) return NVFP4_E_DRIVER;
+  const int64_t ntc = (cols + kTile - 1) / kTile, ntiles = ntc * ((rows + kTile - 1) / kTile);
+  if (ntiles >= (1ll << 31)) return NVFP4_E_LIMIT;
+  const uint32_t grid = ntiles < 2 * sms ? (uint32_t)ntiles : 2u * (uint32_t)sms;
+  if (both) amax_tiles_kernel<true><<<grid, kThreads, kMaxSmemBytes, stream>>>(map, (uint32_t)ntc, (uint32_t)ntiles, signs16, out);
+  else amax_tiles_kernel<false><<<grid, kThreads, kMaxSmemBytes, stream>>>(map, (uint32_t)ntc, (uint32_t)ntiles, signs16, out);
+  return cudaGetLastError() == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
+}
+
 // x [rows, cols] bf16, row pitch ld elements; rows_mode 0 / 1 / 2 = no row-wise output / nearest / stochastic; signs16
 // null = no Hadamard on the transposed output.  counters4 = pitch_r, base_r, pitch_c, base_c.  Arguments have been
 // validated by the caller (quantize.cu): 16-byte aligned pointers, ld % 8 == 0, rows % 16 == 0, and cols % 16 == 0 when
@@ -322,17 +462,8 @@ int launch(const void* x, int64_t rows, int64_t cols, int64_t ld, int rows_mode,
   int sms = 0;
   const int rc = sm_count(sms);
   if (rc != NVFP4_OK) return rc;
-  gemm::EncodeTiledFn enc = gemm::encode_fn();
-  if (enc == nullptr) return NVFP4_E_DRIVER;
   CUtensorMap map;
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 2u};
-  cuuint32_t box[2] = {64u, (cuuint32_t)kTile};
-  cuuint32_t estr[2] = {1u, 1u};
-  if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
-          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return NVFP4_E_DRIVER;
+  if (!make_tile_map(&map, x, rows, cols, ld)) return NVFP4_E_DRIVER;
   Params p;
   p.rows = rows;
   p.cols = cols;

@@ -7,8 +7,8 @@
 //             du = dh * silu(g)
 //
 // The arithmetic is fp32 and the result is rounded to bf16 once.  The maxima are taken over the
-// ROUNDED values, with exactly the operations of amax_plain_kernel / amax_rht_cols_kernel
-// (csrc/quantize.cu), so a quantizer given them produces the bytes it would produce after its own
+// ROUNDED values, with exactly the operations of amax_plain_kernel (csrc/quantize.cu) /
+// amax_tiles_kernel (csrc/quantize_dual.cu), so a quantizer given them produces the bytes it would produce after its own
 // amax pass over the stored tensor.  "RHT_rows" is the 16-point random-sign Hadamard along the ROW
 // (token) dimension in groups of 16 rows: the transform of the wgrad operands (the contraction of
 // dW = dY^T X runs over tokens).
