@@ -101,7 +101,8 @@ class DecoderBlock(nn.Module):
         else:
             q, k, v = self.q(h), self.k(h), self.v(h)
         heads = lambda t, n: t.view(B, T, n, self.head_dim)
-        if rotary.takes(heads(q, self.n_heads), heads(k, self.n_kv), cos, sin):
+        # (grouped heads: the gradients of a group are summed in fp32 on the fp32 copy the torch operations make)
+        if self.n_kv == self.n_heads and rotary.takes(heads(q, self.n_heads), heads(k, self.n_kv), cos, sin):
             q, k = rotary.rotary(heads(q, self.n_heads), heads(k, self.n_kv), cos, sin)
             q, k, v = q.transpose(1, 2), k.transpose(1, 2), split(v, self.n_kv)
         else:

@@ -135,3 +135,19 @@ def test_decoder_block_forward_backward_match_oracle_recipe(fused_norm, tol):
         assert to_ref < tol, (k, to_ref)
         assert to_ref < 0.1 * to_bf16, (k, to_ref, to_bf16)
     assert Q.gemm_status() == 0
+
+
+def test_grouped_heads_sum_their_key_gradients_in_fp32(monkeypatch):
+    """A block with grouped key heads keeps the torch rotary operations: with them the gradients of a group's heads
+    meet on an fp32 copy of the rotated keys, the kernel would add them in bf16."""
+    from nvfp4_sm120_b200 import rotary
+    from nvfp4_sm120_b200.models import DecoderBlock, rotary_tables
+    calls = []
+    real = rotary.rotary
+    monkeypatch.setattr(rotary, "rotary", lambda *a: calls.append(1) or real(*a))
+    cos, sin = rotary_tables(64, 32, "cuda")
+    for n_kv, want in ((2, 0), (4, 1)):
+        blk = DecoderBlock(128, 4, n_kv, 512, True, "cuda")
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            blk(torch.randn(2, 64, 128, device="cuda", requires_grad=True), cos, sin).sum().backward()
+        assert len(calls) == want
