@@ -80,6 +80,19 @@ quant_fused_kernel(const uint16_t* __restrict__ x, uint32_t rows, uint32_t blk_p
       }
     }
   }
+  // Padding of the tiled scale buffer (rows to a multiple of 128, columns to one of 4) reads as zero.  It is written here
+  // while the first loads are under way: a clearing launch in front cost 1.6 us of the GPU and 3 us of the host.
+  {
+    const uint32_t ctiles = (blk_per_row + 3u) >> 2, stride = gridDim.x * THREADS, first = blockIdx.x * THREADS + tid;
+    if ((rows & 127u) != 0) {                    // whole words: word w of a 512-byte tile is row 32 (w & 3) + w / 4 of it
+      uint32_t* last = reinterpret_cast<uint32_t*>(scales) + (uint64_t)(rows >> 7) * ctiles * 128u;
+      for (uint64_t i = first; i < (uint64_t)ctiles * 128u; i += stride)
+        if (((uint32_t)(i & 3u) << 5) + ((uint32_t)(i & 127u) >> 2) >= (rows & 127u)) last[i] = 0u;
+    }
+    if ((blk_per_row & 3u) != 0)                 // the last column tile's missing columns
+      for (uint64_t r = first; r < rows; r += stride)
+        for (uint32_t c = blk_per_row; c < 4u * ctiles; ++c) scales[sf_offset((int64_t)r, c, ctiles)] = 0;
+  }
   if (RHT && tid < 16) sgs[tid] = __ldg(signs16 + tid);
   const bool stamper = blockIdx.x == 0 && tid == 0 && ws != nullptr;
   unsigned long long t_start = 0;
@@ -411,11 +424,6 @@ static int launch_fused(const void* x, int64_t rows, int64_t cols, int64_t ld, i
   const bool known = amax_in != nullptr;
   if (!known && info.coop_ctas < 1) return NVFP4_E_LAUNCH;
   const void* fn = fused_fn(sr, rht != 0, known);
-  const int64_t sm = (rows + 127) / 128 * 128, sk = (cols / 16 + 3) / 4 * 4;
-  if (sm != rows || sk != cols / 16) {
-    if (cudaMemsetAsync(scales, 0, (size_t)(sm * sk), stream) != cudaSuccess) return NVFP4_E_LAUNCH;
-  }
-
   uint32_t rows32 = (uint32_t)rows, bpr = (uint32_t)(cols / 16);
   const uint32_t total = rows32 * bpr;
   uint32_t grid = (uint32_t)(known ? info.sm_count : (info.coop_ctas < info.sm_count ? info.coop_ctas : info.sm_count));
