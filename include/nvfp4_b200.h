@@ -265,8 +265,9 @@ int nvfp4_gemm_fp4out(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pt
 
 /*
  * Kernel choice of nvfp4_gemm for this process: 0 = automatic (the default), 1 = always the
- * one-CTA 128x256 kernel, 2 = always the persistent two-CTA 256x256 kernel.  For tuning and tests;
- * results are the same to rounding of the accumulation order.  No counterpart in the reference.
+ * one-CTA kernel (128 rows x 64 / 128 / 256 columns, a tile shared by up to eight CTAs), 2 = always the
+ * persistent two-CTA kernel (256 rows x 128 / 192 / 256 columns).  For tuning and tests; results are
+ * the same bits, but for tiles shared by several CTAs, whose partial sums are added in a fixed order.  No counterpart in the reference.
  */
 int nvfp4_gemm_set_mode(int mode);
 
@@ -363,7 +364,7 @@ int nvfp4_rotary_bf16(const void* q, void* q_out, int q_heads, const void* k, vo
  *   wait_limit_ns                    the limit (0 = the default, 2 s)
  *   quantizer_extra_arrivals         the quantizer's grid barrier expects this many arrivals more
  *                                    than the grid has CTAs, so it can only run out (code 1)
- *   gemm_drop_first_scale_arrival    != 0: the scale-factor warps never announce K slice 0, so the
+ *   gemm_drop_first_scale_arrival    != 0: the MMA issuer waits for an arrival that never comes, so the
  *                                    MMA issuer's first wait runs out (code 2) and every role leaves
  * nvfp4_test_hooks(0, 0, 0) restores normal operation.  No GPU fault, trap or endless loop is
  * involved: the kernels return through their documented give-up path.  No counterpart in the
