@@ -145,7 +145,15 @@ __global__ void __launch_bounds__(512) amax_plain_kernel(const uint16_t* __restr
     return __ldg(reinterpret_cast<const uint4*>(x + r * ld) + cv);
   };
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  // four 16-byte loads per thread in flight: one per thread leaves the memory system half idle
+  // Eight 16-byte loads per thread in flight and one wave of four CTAs per SM: 8192 x 4096 out of HBM 21.4 -> 17.1 us with
+  // the clearing of the word, 4096 x 14336 25.2 -> 22.9 (four loads and up to eight CTAs per SM in turn before).
+  for (; i + 7 * stride < total; i += 8 * stride) {
+    uint4 q[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) q[u] = load(i + u * stride);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) fold(q[u]);
+  }
   for (; i + 3 * stride < total; i += 4 * stride) {
     const uint4 q0 = load(i), q1 = load(i + stride), q2 = load(i + 2 * stride), q3 = load(i + 3 * stride);
     fold(q0); fold(q1); fold(q2); fold(q3);
@@ -497,7 +505,7 @@ extern "C" int nvfp4_amax_bf16(const void* x, int64_t rows, int64_t cols, int64_
   if (!rht) {
     if ((cols & 7) != 0) return NVFP4_E_SHAPE;
     const int vpr = (int)(cols >> 3);
-    amax_plain_kernel<<<grid_for(rows * vpr, 512 * 4, 148 * 8), 512, 0, stream>>>(xp, rows, vpr, ld, amax);
+    amax_plain_kernel<<<grid_for(rows * vpr, 512 * 8, 148 * 4), 512, 0, stream>>>(xp, rows, vpr, ld, amax);
   } else if (!transpose) {
     if ((cols & 15) != 0) return NVFP4_E_SHAPE;
     const int bpr = (int)(cols >> 4);
