@@ -16,8 +16,7 @@
 // x is read twice, the second time from L2 (a 16-row slab is at most 512 KiB).
 // Backward: dx = rstd * (g*w - xhat * mean(g*w*xhat)), dw = sum over rows of g * xhat, one CTA per
 // 32 rows, dw leaves the CTA as one atomic per column.
-#include "common.cuh"
-#include "nvfp4_b200.h"
+#include "quantize_common.cuh"
 
 namespace nvfp4 {
 namespace rmsnorm {
@@ -98,13 +97,10 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const void* __restrict
   }
   __syncthreads();
   // ---- phase B
-  float sg[16];
+  uint32_t sm[16];                                       // sign-flip masks of the 16 rows
   if (rht) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float4 s = __ldg(reinterpret_cast<const float4*>(signs16) + i);
-      sg[4 * i] = s.x; sg[4 * i + 1] = s.y; sg[4 * i + 2] = s.z; sg[4 * i + 3] = s.w;
-    }
+    for (int i = 0; i < 16; ++i) sm[i] = __ldg(signs16 + i) < 0.0f ? 0x80000000u : 0u;
   }
   const int cc = (threadIdx.x & 63) * 8;
   float m_plain = 0.0f, m_rht = 0.0f;
@@ -126,7 +122,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const void* __restrict
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           hw[q] = pack_bf16x2((v[2 * q] * rs) * wv[2 * q], (v[2 * q + 1] * rs) * wv[2 * q + 1]);
-          m_plain = fmaxf(m_plain, fmaxf(fabsf(bf16_lo(hw[q])), fabsf(bf16_hi(hw[q]))));
+          m_plain = fused::max3_abs(m_plain, bf16_lo(hw[q]), bf16_hi(hw[q]));
         }
         h4 = make_uint4(hw[0], hw[1], hw[2], hw[3]);
         *reinterpret_cast<uint4*>(h + r * cols + c0 + cc) = h4;
@@ -136,17 +132,20 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const void* __restrict
     if (rht) {
       __syncthreads();
       if (c0 + 2 * (int64_t)threadIdx.x < cols) {
-        float v0[16], v1[16];
+        float v0[16], v1[16];                              // two columns in the lanes of packed fp32 instructions
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const uint32_t t = tile[i * kPitchWords + threadIdx.x];
-          v0[i] = bf16_lo(t) * sg[i];
-          v1[i] = bf16_hi(t) * sg[i];
+          v0[i] = __uint_as_float((t << 16) + sm[i]);
+          v1[i] = __uint_as_float((t & 0xffff0000u) ^ sm[i]);
         }
-        hadamard16_inplace(v0);
-        hadamard16_inplace(v1);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) m_rht = fmaxf(m_rht, fmaxf(fabsf(v0[i]), fabsf(v1[i])));
+        for (int s = 1; s < 16; s <<= 1) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if ((i & s) == 0) fused::addsub2(v0[i], v1[i], v0[i | s], v1[i | s]);
+        }
+        m_rht = fmaxf(m_rht, 0.25f * fmaxf(fused::max_abs16(v0), fused::max_abs16(v1)));
       }
       __syncthreads();
     }
