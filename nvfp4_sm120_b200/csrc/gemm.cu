@@ -240,7 +240,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const int quad = warp & 3;                                   // TMEM lanes 32*quad .. +31
     bool ok = true;
     if (ok && lane == 0) {
-      ok = mbar_wait_relaxed(acc_bar, 0, abort_flag);
+      ok = mbar_wait(acc_bar, 0, abort_flag);
       if (!ok) raise(abort_flag, p.status, kErrEpilogueWait);
     }
     ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;

@@ -59,20 +59,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
   }
 }
-// The same for a long wait whose end is not urgent: sleeps between polls so that the waiting lane
-// does not take issue slots from the warps of its scheduler that feed the tensor pipe.
-__device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = global_ns(), limit = wait_limit_of(abort_flag);
-  for (uint32_t i = 1;; ++i) {
-    __nanosleep(64);
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 63u) == 0u) {
-      if (*abort_flag != 0) return false;
-      if (global_ns() - t0 > limit) return false;
-    }
-  }
-}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"

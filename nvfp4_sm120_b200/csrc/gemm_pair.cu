@@ -256,12 +256,13 @@ gemm3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
   } else {
     // ------------------------------ epilogue ------------------------------
     // Two warps per 32-lane quarter of tensor memory, 128 accumulator columns each (the second one 64 of a 192-wide
-    // tile, both 64 of a 128-wide one).  For bf16 output a warp pulls its slab into registers as packed bf16 (64
-    // registers), signals "accumulator read" -- with one accumulator the MMA issuer starts the next tile about 600
-    // cycles after the last MMA of this one -- and only then writes the slab out at leisure, under the next tile's
-    // main loop: swizzled 32 x 128-byte box in shared memory -> TMA store, which writes whole lines and clips at the
-    // matrix edge.  fp32 output (128 registers would not fit) goes box by box and signals after its last
-    // tensor-memory load.
+    // tile, both 64 of a 128-wide one).  A warp pulls its whole slab into registers with loads that are all under way at
+    // once, signals "accumulator read" -- the MMA issuer goes on with the next tile -- and only then converts and writes
+    // the slab out at leisure, under the next tile's main loop: swizzled 32 x 128-byte box in shared memory -> TMA store,
+    // which writes whole lines and clips at the matrix edge.  Signalling behind the conversion (bf16) or behind the third
+    // box (fp32) and polling for the accumulator with sleeps cost, us: 4096 x 28672 x 4096 fp32 222 -> 212, 4096 x 14336 x
+    // 4096 fp32 119.7 -> 113.6, bf16 96.7 -> 94.2, 4096^3 bf16 31.4 -> 30.4.  A second box per warp at the price of the fifth
+    // stage made 256-wide tiles 6-9 % slower.
     const int quad = warp & 3, second = (warp - kEpiWarp0) >> 2;
     const int c_base = S::kSplitCol * second, n_cols = second ? TN - S::kSplitCol : S::kSplitCol;
     uint8_t* boxes = out_stage + (warp - kEpiWarp0) * (S::kBoxes * 4096);
@@ -292,7 +293,7 @@ gemm3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
       const int64_t col0 = n0 + c_base;
       const int a = i % S::kAcc;
       const uint32_t taddr = tmem_base + a * TN + ((uint32_t)(quad * 32) << 16) + c_base;
-      if (lane == 0) ok = mbar_wait_relaxed(acc_full(a), (uint32_t)(i / S::kAcc) & 1u, abort_flag);
+      if (lane == 0) ok = mbar_wait(acc_full(a), (uint32_t)(i / S::kAcc) & 1u, abort_flag);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) { if (lane == 0) raise(abort_flag, p.status, kErrEpilogueWait); break; }
       tc_fence_after();
@@ -300,34 +301,52 @@ gemm3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
         release_accumulator(a);
         continue;
       }
-      if (p.tma_store && !p.out_f32) {
-        uint32_t packed[64];
+      if (p.tma_store) {
+        uint32_t acc[S::kSplitCol / 32][32];
 #pragma unroll
-        for (int ch = 0; ch < S::kSplitCol / 32; ++ch) {
-          if (32 * ch >= n_cols) break;                           // uniform across the warp
-          uint32_t r[32];
-          tc_ld_32x32b_x32(taddr + 32 * ch, r);
-          tc_wait_ld();
-          if (p.d_amax_out != nullptr) track_amax(p, r, alpha, row0 + lane, col0 + 32 * ch, mbits);
+        for (int ch = 0; ch < S::kSplitCol / 32; ++ch)
+          if (32 * ch < n_cols) tc_ld_32x32b_x32(taddr + 32 * ch, acc[ch]);
+        tc_wait_ld();
+        release_accumulator(a);
+        if (p.d_amax_out != nullptr) {
 #pragma unroll
-          for (int q = 0; q < 16; ++q) {
-            __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[2 * q]) * alpha, __uint_as_float(r[2 * q + 1]) * alpha);
-            packed[16 * ch + q] = *reinterpret_cast<uint32_t*>(&h);
+          for (int ch = 0; ch < S::kSplitCol / 32; ++ch)
+            if (32 * ch < n_cols) track_amax(p, acc[ch], alpha, row0 + lane, col0 + 32 * ch, mbits);
+        }
+        if (!p.out_f32) {
+#pragma unroll
+          for (int b = 0; b < S::kSplitCol / 64; ++b) {
+            if (64 * b >= n_cols || col0 + 64 * b >= p.N) break;  // uniform across the warp
+            uint32_t packed[32];
+#pragma unroll
+            for (int q = 0; q < 32; ++q) {
+              const uint32_t* r = &acc[2 * b + (q >> 4)][2 * (q & 15)];
+              __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[0]) * alpha, __uint_as_float(r[1]) * alpha);
+              packed[q] = *reinterpret_cast<uint32_t*>(&h);
+            }
+            box_free();
+            uint8_t* rowp = boxes + which * 4096 + lane * 128;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<uint4*>(rowp + (((uint32_t)j ^ sw) << 4)) =
+                  make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
+            send_box(col0 + 64 * b, row0);
+          }
+        } else {
+#pragma unroll
+          for (int ch = 0; ch < S::kSplitCol / 32; ++ch) {        // fp32: a box is 32 columns
+            if (32 * ch >= n_cols || col0 + 32 * ch >= p.N) break;
+            box_free();
+            uint8_t* rowp = boxes + which * 4096 + lane * 128;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<float4*>(rowp + (((uint32_t)j ^ sw) << 4)) =
+                  make_float4(out_f32(p, acc[ch][4 * j], alpha), out_f32(p, acc[ch][4 * j + 1], alpha),
+                              out_f32(p, acc[ch][4 * j + 2], alpha), out_f32(p, acc[ch][4 * j + 3], alpha));
+            send_box(col0 + 32 * ch, row0);
           }
         }
-        release_accumulator(a);
-#pragma unroll
-        for (int b = 0; b < S::kSplitCol / 64; ++b) {
-          if (64 * b >= n_cols || col0 + 64 * b >= p.N) break;    // uniform across the warp
-          box_free();
-          uint8_t* rowp = boxes + which * 4096 + lane * 128;
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<uint4*>(rowp + (((uint32_t)j ^ sw) << 4)) =
-                make_uint4(packed[32 * b + 4 * j], packed[32 * b + 4 * j + 1], packed[32 * b + 4 * j + 2], packed[32 * b + 4 * j + 3]);
-          send_box(col0 + 64 * b, row0);
-        }
-      } else {
+      } else {                                                    // rows that no tensor map covers, quantized output
         const int64_t n_left = p.N - col0;
         const int chunks = n_left >= n_cols ? n_cols / 32 : (int)((n_left + 31) / 32);
 #pragma unroll 1
@@ -337,18 +356,7 @@ gemm3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
           tc_wait_ld();
           if (ch == chunks - 1) release_accumulator(a);
           if (p.d_amax_out != nullptr) track_amax(p, r, alpha, row0 + lane, col0 + 32 * ch, mbits);
-          if (!p.tma_store) {
-            if (row0 + lane < p.M) store_row_chunk(p, row0 + lane, col0 + 32 * ch, r, alpha);
-            continue;
-          }
-          box_free();                                             // fp32: a box is 32 columns
-          uint8_t* rowp = boxes + which * 4096 + lane * 128;
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<float4*>(rowp + (((uint32_t)j ^ sw) << 4)) =
-                make_float4(out_f32(p, r[4 * j], alpha), out_f32(p, r[4 * j + 1], alpha), out_f32(p, r[4 * j + 2], alpha),
-                            out_f32(p, r[4 * j + 3], alpha));
-          send_box(col0 + 32 * ch, row0);
+          if (row0 + lane < p.M) store_row_chunk(p, row0 + lane, col0 + 32 * ch, r, alpha);
         }
       }
     }
