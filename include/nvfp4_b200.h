@@ -54,6 +54,8 @@ const char* nvfp4_status_string(int code); /* host string, static storage */
  * rht != 0: the maximum is taken AFTER the 16-point random-sign Hadamard transform of every
  * 16-element block (signs16: 16 floats of +-1), blocks running along the columns
  * (transpose == 0) or along the rows (transpose != 0).
+ * A NaN (an element, or a value after the transform) does not count, an infinity does: the rule of
+ * every entry point here that finds a maximum.
  * Replaces `tf.abs().amax()` of quant_nvfp4 (nvfp4_gemm.py:34-36) and the bf16 amax of
  * quant_nvfp4_cuda (nvfp4_cuda.py:170).  A tensor sharded over several GPUs calls this on the
  * local shard, max-reduces the word across ranks, then calls nvfp4_quantize_bf16.

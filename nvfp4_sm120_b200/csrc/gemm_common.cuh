@@ -162,7 +162,7 @@ __device__ __forceinline__ void raise(volatile int* abort_flag, int32_t* status,
 
 
 // Running maximum of |D| over the elements this thread stores, kept as the bit pattern of a
-// non-negative float (unsigned order = numeric order, and a NaN stays on top).  32 accumulator columns
+// non-negative float (unsigned order = numeric order; a NaN does not count).  32 accumulator columns
 // of one output row per call; rows and columns outside the matrix do not count.
 __device__ __forceinline__ void track_amax(const Params& p, const uint32_t (&r)[32], float alpha, int64_t row,
                                            int64_t col, uint32_t& mbits) {
@@ -173,8 +173,7 @@ __device__ __forceinline__ void track_amax(const Params& p, const uint32_t (&r)[
   for (int j = 0; j < 32; ++j) {
     float v = __uint_as_float(r[j]) * alpha;
     if (!p.out_f32) v = __bfloat162float(__float2bfloat16_rn(v));
-    const uint32_t b = __float_as_uint(v) & 0x7fffffffu;
-    if (j < n) mbits = max(mbits, b);
+    if (j < n) mbits = __float_as_uint(fmaxf(__uint_as_float(mbits), fabsf(v)));
   }
 }
 // one atomic per warp and kernel

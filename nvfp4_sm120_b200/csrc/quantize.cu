@@ -125,18 +125,14 @@ __device__ __forceinline__ void cta_max_to(float* addr, float v, int slot = 0) {
 // ---------------------------------------------------------------------------------------
 // amax kernels
 // ---------------------------------------------------------------------------------------
-// plain |x| maximum: 16-byte loads, max taken on the bf16 bit patterns (sign cleared)
+// plain |x| maximum: 16-byte loads, max of packed bf16 magnitudes
 __global__ void __launch_bounds__(512) amax_plain_kernel(const uint16_t* __restrict__ x, int64_t rows,
                                                          int vec_per_row, int64_t ld,
                                                          float* __restrict__ amax) {
   const int64_t total = rows * vec_per_row;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   uint32_t m = 0;
-  auto fold = [&](const uint4& q) {
-    const uint32_t k = 0x7fff7fffu;
-    const uint32_t a = __vimax3_u16x2(q.x & k, q.y & k, q.z & k);
-    m = __vimax3_u16x2(a, q.w & k, m);                 // both 16-bit halves of m carry a running maximum
-  };
+  auto fold = [&](const uint4& q) { m = fused::max_abs_word(m, q); };   // both halves of m carry a running maximum
   const bool flat = ld == (int64_t)vec_per_row * 8;      // contiguous rows: no division per load
   auto load = [&](int64_t i) {
     if (flat) return __ldg(reinterpret_cast<const uint4*>(x) + i);
@@ -159,8 +155,7 @@ __global__ void __launch_bounds__(512) amax_plain_kernel(const uint16_t* __restr
     fold(q0); fold(q1); fold(q2); fold(q3);
   }
   for (; i < total; i += stride) fold(load(i));
-  m = max(m & 0xffffu, m >> 16);
-  cta_max_to(amax, __uint_as_float(m << 16));
+  cta_max_to(amax, fused::max_abs_value(m));
 }
 
 // eight fp32 values -> eight packed bf16, round to nearest even
@@ -186,10 +181,9 @@ __global__ void __launch_bounds__(512) round_amax_kernel(const float* __restrict
     return reinterpret_cast<const float4*>(x + r * ld) + 2 * (i - r * vec_per_row);
   };
   auto fold = [&](int64_t i, const float4& a, const float4& b) {
-    const uint32_t k = 0x7fff7fffu;
     const uint4 q = round8(a, b);
     reinterpret_cast<uint4*>(out)[i] = q;
-    m = __vimax3_u16x2(__vimax3_u16x2(q.x & k, q.y & k, q.z & k), q.w & k, m);
+    m = fused::max_abs_word(m, q);
   };
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (; i + stride < total; i += 2 * stride) {
@@ -202,8 +196,7 @@ __global__ void __launch_bounds__(512) round_amax_kernel(const float* __restrict
     const float4* p = src(i);
     fold(i, __ldg(p), __ldg(p + 1));
   }
-  m = max(m & 0xffffu, m >> 16);
-  cta_max_to(amax, __uint_as_float(m << 16));
+  cta_max_to(amax, fused::max_abs_value(m));
 }
 
 // maximum after the Hadamard transform, blocks along the columns: one thread per block
@@ -373,11 +366,7 @@ __global__ void __launch_bounds__(256) round_amax_both_kernel(const float* __res
     if (t.r_base + 16 * j >= rows) break;                  // uniform over the CTA
     wide_stage(tile, t, nxt);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint32_t kk = 0x7fff7fffu;
-      mp = __vimax3_u16x2(mp, nxt[k].x & kk, nxt[k].y & kk);
-      mp = __vimax3_u16x2(mp, nxt[k].z & kk, nxt[k].w & kk);
-    }
+    for (int k = 0; k < 4; ++k) mp = fused::max_abs_word(mp, nxt[k]);
     if (j + 1 < 4) wide_fetch_round(x, rows, cols, ld, t, j + 1, rounded, nxt);
     __syncthreads();
     if (t.mine) {
@@ -394,8 +383,7 @@ __global__ void __launch_bounds__(256) round_amax_both_kernel(const float* __res
     }
     __syncthreads();
   }
-  mp = max(mp & 0xffffu, mp >> 16);
-  cta_max_to(out, __uint_as_float(mp << 16), 0);
+  cta_max_to(out, fused::max_abs_value(mp), 0);
   cta_max_to(out + 1, m, 1);
 }
 

@@ -74,6 +74,26 @@ __device__ __forceinline__ float amax_packed8(const uint32_t (&w)[8]) {
   return __uint_as_float(max(m << 16, m & 0xffff0000u));
 }
 
+// Magnitudes of packed bf16 pairs: the larger one per half, its sign bit meaningless.  A NaN does not count beside a number.
+__device__ __forceinline__ uint32_t max_abs_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+// m with the eight values of a 16-byte word folded in (m starts at 0, so it stays a number)
+__device__ __forceinline__ uint32_t max_abs_word(uint32_t m, const uint4& q) {
+  return max_abs_bf16x2(m, max_abs_bf16x2(max_abs_bf16x2(q.x, q.y), max_abs_bf16x2(q.z, q.w)));
+}
+__device__ __forceinline__ float max_abs_value(uint32_t m) {
+  return __uint_as_float(max((m << 16) & 0x7fff0000u, m & 0x7fff0000u));
+}
+// What a block adds to the per-tensor maximum: its maximum, and if it holds a NaN that of its numbers.
+__device__ __forceinline__ float amax_of_numbers(float amax_b, const uint32_t (&w)[8]) {
+  if (__builtin_expect(amax_b <= __uint_as_float(0x7f800000u), 1)) return amax_b;
+  const uint32_t m = max_abs_word(0u, make_uint4(w[0], w[1], w[2], w[3]));
+  return max_abs_value(max_abs_word(m, make_uint4(w[4], w[5], w[6], w[7])));
+}
+
 // max(m, |a|, |b|) as one three-input instruction (a NaN operand does not count, as with fmaxf)
 __device__ __forceinline__ float max3_abs(float m, float a, float b) {
   float r;

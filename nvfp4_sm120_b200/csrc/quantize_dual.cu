@@ -340,10 +340,7 @@ amax_tiles_kernel(const __grid_constant__ CUtensorMap map_x, uint32_t ntc, uint3
         v0[k] = __uint_as_float((w[e] << 16) + sm[e]);
         v1[k] = __uint_as_float((w[e] & 0xffff0000u) ^ sm[e]);
       }
-      if (BOTH) {
-        const uint32_t kk = 0x7fff7fffu;
-        mp = __vimax3_u16x2(__vimax3_u16x2(mp, w[0] & kk, w[1] & kk), w[2] & kk, w[3] & kk);
-      }
+      if (BOTH) mp = fused::max_abs_word(mp, make_uint4(w[0], w[1], w[2], w[3]));
     }
 #pragma unroll
     for (int s = 1; s < 16; s <<= 1) {
@@ -359,9 +356,8 @@ amax_tiles_kernel(const __grid_constant__ CUtensorMap map_x, uint32_t ntc, uint3
       fetch(i + kMaxSlots);
     }
   }
-  const float plain = __uint_as_float(max(mp & 0xffffu, mp >> 16) << 16);
-  // a NaN has the largest bit pattern: the plain maximum compares bits, as the plain kernel's does
-  const uint32_t plain_bits = __reduce_max_sync(0xffffffffu, __float_as_uint(plain));
+  // neither maximum can be a NaN (NaNs do not count), so they order like their bits
+  const uint32_t plain_bits = __reduce_max_sync(0xffffffffu, __float_as_uint(fused::max_abs_value(mp)));
   m = warp_max(m * 0.25f);                                                // the transform is butterfly / 4
   if (lane == 0) { part[warp] = m; part[16 + warp] = __uint_as_float(plain_bits); }
   __syncthreads();

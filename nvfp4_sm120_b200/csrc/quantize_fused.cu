@@ -130,7 +130,7 @@ quant_fused_kernel(const uint16_t* __restrict__ x, uint32_t rows, uint32_t blk_p
     }
     const float a = amax_packed8(w);
     if (i - b0 < (uint32_t)kTabBlocks) amax_tab[i - b0] = (uint16_t)(__float_as_uint(a) >> 16);
-    return a;
+    return amax_of_numbers(a, w);
   };
   // the streamed head, kBatch blocks per thread in flight before any of them is consumed
   for (uint32_t i = b0 + tid; i < s0 && !known; i += kBatch * THREADS) {

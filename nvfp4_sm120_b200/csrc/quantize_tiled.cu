@@ -244,6 +244,7 @@ quant_tiled_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
         } else {
           a = amax_packed8(w[e]);
           if (c < (uint32_t)(kTabTiles / 2)) tp[e * kHalfThreads] = (uint16_t)(__float_as_uint(a) >> 16);
+          a = amax_of_numbers(a, w[e]);
         }
         if (e == 0 || two) m = fmaxf(m, a);
       }
