@@ -237,8 +237,7 @@ int nvfp4_gemm(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pts,
  * nvfp4_gemm that also leaves max|D| in *d_amax_out (fp32 device word; the call zeroes it on the
  * stream first): the maximum over the stored output after its rounding to the output type, i.e.
  * what nvfp4_amax_bf16 would find by reading D again.  A quantizer that takes D next
- * (nvfp4_quantize_fused_bf16 with this word as amax_in) then needs one pass, not two.  The K split
- * of small fp32 outputs is not used with this entry point.
+ * (nvfp4_quantize_bf16 with this word) then needs one pass, not two.  D is the D of nvfp4_gemm, bit for bit.
  * Replaces the `tf.abs().amax()` pass of quant_nvfp4 (nvfp4_gemm.py:34-36) over a GEMM output, e.g.
  * between `up` and `down` at nvfp4_train.py:111-123; the quantization overhead it removes is the one
  * the reference names at README.md:80-83.

@@ -68,6 +68,7 @@ __device__ __forceinline__ void sum_partials(const Params& p, uint32_t smem_base
   constexpr int kVecs = TN / S / 4, kBatch = 8 / S;
   const int rows = (int)min((int64_t)kTileM, p.M - m0), items = rows * kVecs;
   const float alpha = __ldg(p.a_pts) * __ldg(p.b_pts);
+  float m = 0.0f;                                               // max|D| of what this thread stores
   for (int i0 = threadIdx.x; i0 < items; i0 += kThreads * kBatch) {
     float4 v[kBatch][S];
 #pragma unroll
@@ -90,6 +91,8 @@ __device__ __forceinline__ void sum_partials(const Params& p, uint32_t smem_base
       float o[4] = {s.x * alpha, s.y * alpha, s.z * alpha, s.w * alpha};
       if (p.round_bf16)
         for (int j = 0; j < 4; ++j) o[j] = __bfloat162float(__float2bfloat16_rn(o[j]));
+      if (p.d_amax_out != nullptr)                              // (columns outside hold zeros)
+        for (int j = 0; j < 4; ++j) m = fmaxf(m, fabsf(p.out_f32 ? o[j] : __bfloat162float(__float2bfloat16_rn(o[j]))));
       const int64_t d = (m0 + r) * p.ldd + col;
       const bool vec = col + 4 <= p.N && (p.ldd & 3) == 0;
       if (p.out_f32) {
@@ -110,6 +113,46 @@ __device__ __forceinline__ void sum_partials(const Params& p, uint32_t smem_base
       }
     }
   }
+  flush_amax(p, __float_as_uint(m), threadIdx.x & 31);
+}
+// The same share as NVFP4: a thread takes one block of 16 columns.  The sums are those of sum_partials, in its order, so
+// the bytes are what quantizing its bf16 result gives.
+template <int TN, int S>
+__device__ __forceinline__ void quantize_partials(const Params& p, uint32_t smem_base, uint32_t rank, int64_t m0, int64_t n0) {
+  constexpr int kBlocks = TN / S / 16, kDiv = kBlocks > 0 ? kBlocks : 1;   // none for TN 64, S 8: not launched with this output
+  const float alpha = __ldg(p.a_pts) * __ldg(p.b_pts);
+  const float pts = __fdiv_rn(fmaxf(__ldg(p.d_amax), kAmaxFloor), kGlobalDiv), inv_pts = __fdiv_rn(1.0f, pts);
+  const int64_t col_tiles = ((p.N >> 4) + 3) >> 2;
+  const int items = (int)min((int64_t)kTileM, p.M - m0) * kBlocks;
+  for (int i = threadIdx.x; i < items; i += kThreads) {
+    const int r = i / kDiv, c = ((int)rank * kBlocks + (i - r * kBlocks)) * 16;
+    const int64_t row = m0 + r, col = n0 + c;
+    if (col >= p.N) continue;                                   // N is a multiple of 16: a block is whole or absent
+    const uint32_t at = smem_base + 4u * (uint32_t)(r * Tile<TN>::kPartPitch + c);
+    float4 v[4][S];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int k = 0; k < S; ++k) v[q][k] = load_cluster(at + 16u * q, (uint32_t)k);
+    uint32_t acc[16];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float4 s = v[q][0];
+#pragma unroll
+      for (int k = 1; k < S; ++k) { s.x += v[q][k].x; s.y += v[q][k].y; s.z += v[q][k].z; s.w += v[q][k].w; }
+      acc[4 * q] = __float_as_uint(s.x); acc[4 * q + 1] = __float_as_uint(s.y);
+      acc[4 * q + 2] = __float_as_uint(s.z); acc[4 * q + 3] = __float_as_uint(s.w);
+    }
+    uint32_t lo, hi, sf;
+    quantize_out_block(acc, alpha, pts, inv_pts, lo, hi, sf);
+    *reinterpret_cast<uint2*>(static_cast<uint8_t*>(p.d) + row * (p.N >> 1) + (col >> 1)) = make_uint2(lo, hi);
+    p.d_sf[sf_offset(row, col >> 4, col_tiles)] = (uint8_t)sf;
+  }
+}
+template <int TN, int S>
+__device__ __forceinline__ void finish_shared_tile(const Params& p, uint32_t smem_base, uint32_t rank, int64_t m0, int64_t n0) {
+  if (p.out_fp4) quantize_partials<TN, S>(p, smem_base, rank, m0, n0);
+  else sum_partials<TN, S>(p, smem_base, rank, m0, n0);
 }
 
 template <int TN>
@@ -285,9 +328,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   __syncthreads();
   if (p.splits > 1) {
     cluster_sync_all();                                          // every partial sum of the tile is in place
-    if (p.splits == 2) sum_partials<TN, 2>(p, base, split, m0, n0);
-    else if (p.splits == 4) sum_partials<TN, 4>(p, base, split, m0, n0);
-    else sum_partials<TN, 8>(p, base, split, m0, n0);
+    if (p.splits == 2) finish_shared_tile<TN, 2>(p, base, split, m0, n0);
+    else if (p.splits == 4) finish_shared_tile<TN, 4>(p, base, split, m0, n0);
+    else finish_shared_tile<TN, 8>(p, base, split, m0, n0);
     cluster_sync_all();                                          // nobody reads this CTA's shared memory any more
   }
   if (warp == 1) {

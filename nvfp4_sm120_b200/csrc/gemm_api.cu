@@ -51,7 +51,7 @@ struct Choice { bool pair; int tile_n, splits; };
 // 768 6.7 / 7.2 (128 x 256), 2048 x 768 x 3072 8.6 / 9.8 (pair 256 x 128), 1000 x 2584 x 7136 17.0 / 18.6 (pair 256 x 192),
 // 256 x 1024 x 8192 8.9 / 14.9 (128 x 64, four CTAs per tile), 64 x 4096 x 14336 12.6 / 22.9 (128 x 128, four),
 // 768 x 768 x 16384 15.3 / 24.7 (128 x 64, two), 8 x 14336 x 4096 11.9 / 12.6 (128 x 256, two).
-static Choice choose(int64_t M, int64_t N, int64_t K, int forced, bool may_split) {
+static Choice choose(int64_t M, int64_t N, int64_t K, int forced) {
   struct Kind { bool pair; int tile_n; float fixed, slice, drain, sum; };
   static const Kind kinds[] = {{true, 256, 5.75f, 0.315f, 1.3f, 0.0f}, {true, 192, 5.35f, 0.31f, 0.85f, 0.0f},
                                {true, 128, 4.75f, 0.29f, 0.6f, 0.0f},  {false, 256, 5.35f, 0.39f, 4.3f, 2.6f},
@@ -64,7 +64,7 @@ static Choice choose(int64_t M, int64_t N, int64_t K, int forced, bool may_split
   for (const Kind& k : kinds) {
     if (forced != 0 && k.pair != (forced == 2)) continue;
     const int64_t rows = k.pair ? 256 : 128, tiles = ((M + rows - 1) / rows) * ((N + k.tile_n - 1) / k.tile_n);
-    for (int log_s = 0; log_s < (k.pair || !may_split ? 1 : 4); ++log_s) {
+    for (int log_s = 0; log_s < (k.pair ? 1 : 4); ++log_s) {
       const int s = 1 << log_s;
       const int64_t per = (slices + s - 1) / s, cap = k.pair ? 74 : caps[log_s];
       if (s > 1 && (tiles * s > cap || per * (s - 1) >= slices)) break;      // one wave, and work for every CTA
@@ -95,8 +95,10 @@ static int gemm_any(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pts,
     if (cudaMemsetAsync(d_amax_out, 0, sizeof(float), stream) != cudaSuccess) return NVFP4_E_LAUNCH;
   }
   const int forced = g_gemm_mode.load(std::memory_order_relaxed);
-  // (a shared tile is stored by the cluster's sum: no maximum, no quantized output there)
-  const Choice pick = choose(M, N, K, forced, !fp4_out && d_amax_out == nullptr);
+  // One choice for every form of output, so that all of them hold the same sums.  (A quantized output wants whole blocks
+  // of 16 columns in a CTA's share: 64 columns over eight CTAs become 128, the same shares of K.)
+  Choice pick = choose(M, N, K, forced);
+  if (fp4_out && pick.tile_n < 16 * pick.splits) pick.tile_n = 128;
   Params p{a_sf, b_sf, a_pts, b_pts, d, M, N, K, ldd, out_dtype == NVFP4_OUT_F32 ? 1 : 0, status, pick.splits, 0,
            g_gemm_wait_ns.load(std::memory_order_relaxed), g_gemm_drop_arrival.load(std::memory_order_relaxed),
            d_sf, d_amax, fp4_out ? 1 : 0, round_bf16, d_amax_out};
