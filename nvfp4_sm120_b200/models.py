@@ -77,6 +77,10 @@ class DecoderBlock(nn.Module):
         # its output (one sign vector serves q, k, v; each consumer checks it against its own)
         self.fused_norm = bool(use_fp4) and all(isinstance(m, FP4Linear) for m in (self.q, self.k, self.v, self.up))
 
+        # the rotary kernel likewise; dense projections keep the torch operations, which torch.func transforms,
+        # forward-mode differentiation and tracing take (an FP4Linear takes none of them)
+        self.fused_rotary = bool(use_fp4) and isinstance(self.q, FP4Linear) and isinstance(self.k, FP4Linear)
+
     def _norm(self, norm, x, consumer):
         """norm(x) -> (h, maxima or None): the fused kernel when the consumers are FP4Linear on the GPU."""
         if (self.fused_norm and x.is_cuda and x.dtype in (torch.float32, torch.bfloat16) and x.shape[-1] % 8 == 0
@@ -102,7 +106,8 @@ class DecoderBlock(nn.Module):
             q, k, v = self.q(h), self.k(h), self.v(h)
         heads = lambda t, n: t.view(B, T, n, self.head_dim)
         # (grouped heads: the gradients of a group are summed in fp32 on the fp32 copy the torch operations make)
-        if self.n_kv == self.n_heads and rotary.takes(heads(q, self.n_heads), heads(k, self.n_kv), cos, sin):
+        if (self.fused_rotary and self.n_kv == self.n_heads
+                and rotary.takes(heads(q, self.n_heads), heads(k, self.n_kv), cos, sin)):
             q, k = rotary.rotary(heads(q, self.n_heads), heads(k, self.n_kv), cos, sin)
             q, k, v = q.transpose(1, 2), k.transpose(1, 2), split(v, self.n_kv)
         else:

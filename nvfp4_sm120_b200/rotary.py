@@ -10,28 +10,31 @@ from .quant import _stream
 
 
 class RotaryFn(torch.autograd.Function):
-    """(q [B, T, Hq, D], k [B, T, Hk, D], cos, sin [T, D / 2]) -> both rotated, bf16, same layout."""
+    """(q [B, T, Hq, D], k [B, T, Hk, D], cos, sin [T, D / 2]) -> both rotated, bf16, same layout.  transposed: by the
+    transposed rotation.  The operation is linear and its gradient is the other of the two, so it can be differentiated
+    any number of times."""
 
     @staticmethod
-    def forward(ctx, q, k, cos, sin):
+    def forward(ctx, q, k, cos, sin, transposed):
         ctx.save_for_backward(cos, sin)
-        return _rotate(q, k, cos, sin, 0)
+        ctx.transposed = transposed
+        return _rotate(q, k, cos, sin, transposed)
 
     @staticmethod
     def backward(ctx, gq, gk):
-        cos, sin = ctx.saved_tensors
-        gq, gk = _rotate(gq.to(torch.bfloat16), gk.to(torch.bfloat16), cos, sin, 1)
-        return gq, gk, None, None
+        args = gq.to(torch.bfloat16), gk.to(torch.bfloat16), *ctx.saved_tensors, not ctx.transposed
+        gq, gk = RotaryFn.apply(*args) if torch.is_grad_enabled() else _rotate(*args)
+        return gq, gk, None, None, None
 
 
-def _rotate(q, k, cos, sin, backward):
+def _rotate(q, k, cos, sin, transposed):
     q, k = _rows(q), _rows(k)
     dev = _lib.cuda_device_of(q, k, cos, sin)
     B, T, hq, D = q.shape
     qo, ko = torch.empty_like(q), torch.empty_like(k)
     with torch.cuda.device(dev):                   # the C side launches on the current device
         code = _lib.lib().nvfp4_rotary_bf16(q.data_ptr(), qo.data_ptr(), hq, k.data_ptr(), ko.data_ptr(), k.shape[2], B * T,
-                                            T, D, cos.data_ptr(), sin.data_ptr(), backward, _stream(dev))
+                                            T, D, cos.data_ptr(), sin.data_ptr(), int(transposed), _stream(dev))
     _lib.check(code, "nvfp4_rotary_bf16")
     return qo, ko
 
@@ -54,4 +57,4 @@ def takes(q, k, cos, sin):
 def rotary(q, k, cos, sin):
     """q [B, T, Hq, D] and k [B, T, Hk, D] rotated by the tables [1, 1, T, D / 2]."""
     T, half = cos.shape[2:]
-    return RotaryFn.apply(q, k, _rows(cos.reshape(T, half)), _rows(sin.reshape(T, half)))
+    return RotaryFn.apply(q, k, _rows(cos.reshape(T, half)), _rows(sin.reshape(T, half)), False)

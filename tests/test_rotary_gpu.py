@@ -39,3 +39,43 @@ def test_calls_that_keep_the_torch_operations():
         assert not rotary.takes(q.bfloat16(), q.bfloat16(), cos[..., :8], sin[..., :8])
     with torch.autocast("cuda", dtype=torch.float16):
         assert not rotary.takes(q.bfloat16(), q.bfloat16(), cos, sin)
+
+
+def _hessian_vector_product(block, x, v, cos, sin):
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+    with sdpa_kernel(SDPBackend.MATH), torch.autocast("cuda", dtype=torch.bfloat16):
+        loss = block(x, cos, sin).square().sum()
+    g, = torch.autograd.grad(loss, x, create_graph=True)
+    return torch.autograd.grad((g * v).sum(), x)[0]
+
+
+def test_dense_blocks_have_second_derivatives(monkeypatch):
+    """Without FP4 linears everything in a block is differentiable twice, and takes torch.func transforms."""
+    from nvfp4_sm120_b200 import models, rotary
+    torch.manual_seed(3)
+    block = models.DecoderBlock(64, 2, 2, 128, False, "cuda")
+    x, v = torch.randn(1, 16, 64, device="cuda", requires_grad=True), torch.randn(1, 16, 64, device="cuda")
+    cos, sin = models.rotary_tables(16, 32, "cuda")
+    got = _hessian_vector_product(block, x, v, cos, sin)
+
+    def energy(t):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            return block(t, cos, sin).square().sum()
+
+    assert torch.func.grad(energy)(x.detach()).shape == x.shape
+    monkeypatch.setattr(rotary, "takes", lambda *a: False)
+    assert torch.equal(got, _hessian_vector_product(block, x, v, cos, sin))
+
+
+def test_the_kernel_differentiates_twice():
+    """The rotation is linear: the derivative of its backward is the rotation of the direction."""
+    from nvfp4_sm120_b200 import models, rotary
+    cos, sin = models.rotary_tables(8, 32, "cuda")
+    make = lambda: torch.randn(2, 8, 3, 32, device="cuda").bfloat16()
+    q, k = make().requires_grad_(True), make().requires_grad_(True)
+    a, b = rotary.rotary(q, k, cos, sin)
+    ga, gb, u, w = make().requires_grad_(True), make().requires_grad_(True), make(), make()
+    dq, dk = torch.autograd.grad([a, b], [q, k], [ga, gb], create_graph=True)
+    got = torch.autograd.grad([dq, dk], [ga, gb], [u, w])
+    for x, y in zip(got, rotary.rotary(u, w, cos, sin)):
+        assert torch.equal(x, y)
