@@ -145,25 +145,24 @@ void check_matrix(const at::Tensor& t) {
   if (!t.is_cuda()) device_of({&t});
 }
 // rows the kernels can read: unit column stride, a row pitch of 16-byte multiples, a 16-byte aligned start
-at::Tensor as_rows(const at::Tensor& x, int64_t pitch_multiple) {
-  if (x.stride(1) != 1 || x.stride(0) % pitch_multiple != 0 || x.stride(0) < x.size(1) ||
-      reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0)
-    return x.contiguous();
-  return x;
+bool readable_rows(const at::Tensor& x) {
+  return x.stride(1) == 1 && x.stride(0) * x.element_size() % 16 == 0 && x.stride(0) >= x.size(1) &&
+         reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0;
 }
 at::Tensor as_bf16_rows(const at::Tensor& t) {
   check_matrix(t);
-  return as_rows(t.scalar_type() == at::kBFloat16 ? t : t.to(at::kBFloat16), 8);
+  const at::Tensor x = t.scalar_type() == at::kBFloat16 ? t : t.to(at::kBFloat16);
+  return readable_rows(x) ? x : x.contiguous();
 }
 
 // An fp32 matrix whose bf16 rounding and maximum (both maxima with signs: after the Hadamard transform along the rows
-// too) one kernel finds: (bf16 copy, maxima).  For shapes that the kernel takes.
+// too) one kernel finds: (bf16 copy, maxima).  For shapes that the kernel takes and memory it can read as it is: the
+// cast of any other matrix makes an aligned copy, where an fp32 copy in front of this kernel would be a pass more.
 bool can_round(const at::Tensor& t, bool rht) {
   return t.scalar_type() == at::kFloat && t.size(0) > 0 && t.size(1) > 0 && t.size(1) % 8 == 0 &&
-         (!rht || t.size(0) % 16 == 0) && t.size(0) <= 64 * 65535LL;
+         (!rht || t.size(0) % 16 == 0) && t.size(0) <= 64 * 65535LL && readable_rows(t);
 }
-std::pair<at::Tensor, at::Tensor> round_amax(const at::Tensor& t, const at::Tensor* signs) {
-  const at::Tensor x = as_rows(t, 4);
+std::pair<at::Tensor, at::Tensor> round_amax(const at::Tensor& x, const at::Tensor* signs) {
   const c10::Device dev = device_of({&x, signs});
   at::Tensor out = at::empty({x.size(0), x.size(1)}, on(dev, at::kBFloat16));
   at::Tensor maxima = at::empty({signs != nullptr ? 2 : 1}, on(dev, at::kFloat));

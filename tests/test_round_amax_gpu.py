@@ -44,3 +44,19 @@ def test_values_that_are_not_finite(Q):
     a, b = Q.quant_weight_nvfp4(x), Q.quant_weight_nvfp4(x.to(torch.bfloat16))
     for u, v in zip(a, b):
         assert torch.equal(u.qdata, v.qdata) and torch.equal(u.scale.view(torch.uint8), v.scale.view(torch.uint8))
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3, 4])
+def test_starts_that_are_not_aligned(Q, offset):
+    """A view into a flat fp32 buffer at any element, as a parameter of a flattened module is."""
+    flat = torch.randn(64 * 96 + 8, device="cuda")
+    x = flat[offset:offset + 64 * 96].view(64, 96)
+    b = x.to(torch.bfloat16)
+    signs = O.signs_from_seed(4).cuda()
+    for u, v in zip(Q.quant_weight_nvfp4(x), Q.quant_weight_nvfp4(b)):
+        assert _same(u, v)
+    for u, v in zip(Q.quant_dual_nvfp4(x, signs), Q.quant_dual_nvfp4(b, signs)):
+        assert _same(u, v)
+    assert _same(Q.quant_nvfp4(x, transpose=True), Q.quant_nvfp4(b, transpose=True))
+    big = torch.randn(2048 * 2048 + 8, device="cuda")[offset:offset + 2048 * 2048].view(2048, 2048)
+    assert _same(Q.quant_nvfp4(big), Q.quant_nvfp4(big.to(torch.bfloat16)))
