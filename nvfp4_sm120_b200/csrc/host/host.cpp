@@ -160,7 +160,7 @@ at::Tensor as_bf16_rows(const at::Tensor& t) {
 // cast of any other matrix makes an aligned copy, where an fp32 copy in front of this kernel would be a pass more.
 bool can_round(const at::Tensor& t, bool rht) {
   return t.scalar_type() == at::kFloat && t.size(0) > 0 && t.size(1) > 0 && t.size(1) % 8 == 0 &&
-         (!rht || t.size(0) % 16 == 0) && t.size(0) <= 64 * 65535LL && readable_rows(t);
+         (!rht || t.size(0) % 16 == 0) && t.size(0) <= 64 * 65535LL && readable_rows(t) && !t.is_neg();
 }
 std::pair<at::Tensor, at::Tensor> round_amax(const at::Tensor& x, const at::Tensor* signs) {
   const c10::Device dev = device_of({&x, signs});

@@ -60,3 +60,9 @@ def test_starts_that_are_not_aligned(Q, offset):
     assert _same(Q.quant_nvfp4(x, transpose=True), Q.quant_nvfp4(b, transpose=True))
     big = torch.randn(2048 * 2048 + 8, device="cuda")[offset:offset + 2048 * 2048].view(2048, 2048)
     assert _same(Q.quant_nvfp4(big), Q.quant_nvfp4(big.to(torch.bfloat16)))
+
+
+def test_a_negated_view(Q):
+    x = torch.randn(64, 96, device="cuda")
+    for u, v in zip(Q.quant_weight_nvfp4(torch._neg_view(x)), Q.quant_weight_nvfp4(-x)):
+        assert _same(u, v)
