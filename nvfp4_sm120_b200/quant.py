@@ -11,6 +11,7 @@ from .tensor import BLK, NVFP4Tensor
 
 F4_MAX, F8E4M3_MAX, E4M3_EPS = 6.0, 448.0, 0.015625
 
+_M64 = 2 ** 64 - 1   # seeds, offsets and counters are 64-bit words: any integer, modulo 2^64
 _SEED = [0]          # auto-advancing seed of stochastic calls, like nvfp4_cuda.py:154,160-162
 _H_OK = {}           # H tensors already checked to be the Sylvester matrix / 4
 
@@ -93,9 +94,8 @@ def quant_nvfp4(t, stochastic=False, rht=False, H=None, signs=None, seed=None, *
         if stochastic:
             _SEED[0] += 1
     _check_h(H)
-    pitch, base = (-1, 0) if counter is None else (int(counter[0]), int(counter[1]))
-    q, s, pts = _lib.host().quantize(t, bool(stochastic), bool(rht), signs, int(seed) & (2 ** 64 - 1), bool(transpose),
-                                     amax, int(philox_offset), bool(fused), pitch, base)
+    q, s, pts = _lib.host().quantize(t, bool(stochastic), bool(rht), signs, int(seed) & _M64, bool(transpose), amax,
+                                     int(philox_offset) & _M64, bool(fused), [] if counter is None else [int(v) & _M64 for v in counter[:2]])
     return NVFP4Tensor(q, s, BLK, t.dtype, pts, True)
 
 
@@ -132,8 +132,8 @@ def quant_dual_nvfp4(t, signs, amax_rows=None, amax_cols=None, stochastic_rows=F
         if stochastic_cols:
             _SEED[0] += 1
     q_r, s_r, p_r, q_c, s_c, p_c = _lib.host().quantize_dual(
-        t, signs, amax_rows, amax_cols, bool(stochastic_rows), bool(stochastic_cols), int(seed_rows) & (2 ** 64 - 1),
-        int(seed_cols) & (2 ** 64 - 1), int(philox_offset), [] if counters is None else [int(v) for v in counters])
+        t, signs, amax_rows, amax_cols, bool(stochastic_rows), bool(stochastic_cols), int(seed_rows) & _M64, int(seed_cols) & _M64,
+        int(philox_offset) & _M64, [] if counters is None else [int(v) & _M64 for v in counters])
     return (NVFP4Tensor(q_r, s_r, BLK, t.dtype, p_r, True), NVFP4Tensor(q_c, s_c, BLK, t.dtype, p_c, True))
 
 

@@ -256,3 +256,18 @@ def test_shard_counters_reproduce_the_whole_tensor(Q, rht):
     full_tsc = O.unswizzle_scales(full_t.scale.view(torch.uint8).cpu(), 512, 256)
     part_tsc = O.unswizzle_scales(part_t.scale.view(torch.uint8).cpu(), c1 - c0, 256)
     assert torch.equal(part_tsc, full_tsc[c0:c1])
+
+
+def test_offsets_and_counters_are_taken_modulo_2_64(Q):
+    x = torch.randn(32, 64, device="cuda").to(torch.bfloat16)
+    amax = x.abs().max().float().reshape(1)
+    signs = O.signs_from_seed(4).cuda()
+    same = lambda a, b: torch.equal(a.qdata, b.qdata)
+    top = 2 ** 64 - 1
+    assert same(Q.quant_nvfp4(x, True, seed=1, philox_offset=-1), Q.quant_nvfp4(x, True, seed=1, philox_offset=top))
+    assert same(Q.quant_nvfp4(x, True, seed=1, amax=amax, counter=(4, -1)),
+                Q.quant_nvfp4(x, True, seed=1, amax=amax, counter=(4, top)))
+    for offset in (-1, top + 2 ** 64):
+        for a, b in zip(Q.quant_dual_nvfp4(x, signs, None, None, True, True, 1, 2, philox_offset=offset, counters=(4, -1, 2, 0)),
+                        Q.quant_dual_nvfp4(x, signs, None, None, True, True, 1, 2, philox_offset=top, counters=(4, top, 2, 0))):
+            assert same(a, b)
