@@ -157,7 +157,12 @@ class FP4LinearFn(torch.autograd.Function):
                                        x_amax[1:2] if have_both else None)
         else:
             xq = _quant(x2, x_red, amax=None if x_amax is None else x_amax[0:1])
-        if wq_K is None:
+        own_wq_N = None
+        if wq_K is None and grad_on and ctx.needs_input_grad[0] and amax_reduce is None:
+            # both layouts of the weight from one read: fprop's operand now, dgrad's for the backward, which keeps 0.56 B
+            # per weight element until then
+            wq_K, own_wq_N = quant_weight_nvfp4(w)
+        elif wq_K is None:
             wq_K = _quant(w, amax_reduce)
         # y_amax_out: optional fp32 [1] that the fprop GEMM's epilogue fills with max|y| (for a consumer
         # that quantizes y next; only meaningful when y stays bf16, i.e. x is bf16)
@@ -165,11 +170,10 @@ class FP4LinearFn(torch.autograd.Function):
             y = mm_as(xq, wq_K.t(), x.dtype)
         else:
             y = nvfp4_mm(xq, wq_K.t(), torch.bfloat16, amax_out=y_amax_out).to(x.dtype)
-        if xtq is None:
-            ctx.save_for_backward(x2, w)
-        else:
-            ctx.save_for_backward(w, xtq.qdata, xtq.scale, xtq.per_tensor_scale)
-        ctx.have_xtq = xtq is not None
+        # everything made here goes through autograd's saved tensors (a wq_N that came in belongs to the caller's cache)
+        parts = lambda t: () if t is None else (t.qdata, t.scale, t.per_tensor_scale)
+        ctx.save_for_backward(w, x2 if xtq is None else None, *parts(xtq), *parts(own_wq_N))
+        ctx.have_xtq, ctx.have_wq_N = xtq is not None, own_wq_N is not None
         ctx.H, ctx.signs, ctx.xshape, ctx.wq_N = H, signs, x.shape, wq_N
         ctx.amax_reduce, ctx.sharded, ctx.x_amax = amax_reduce, sharded, x_amax
         ctx.x_amax_rht = bool(x_amax_rht)        # False: the Hadamard maximum came from another sign vector
@@ -178,14 +182,13 @@ class FP4LinearFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, gy):
-        if ctx.have_xtq:
-            w, xt_q, xt_s, xt_p = ctx.saved_tensors
-            x2 = None
-            xtq = NVFP4Tensor(xt_q, xt_s, BLK, torch.bfloat16, xt_p, True)
-        else:
-            x2, w = ctx.saved_tensors
-            xtq = None
+        w, x2, *parts = ctx.saved_tensors
+        xtq = None
         H, signs, wq_N, red = ctx.H, ctx.signs, ctx.wq_N, ctx.amax_reduce
+        if ctx.have_xtq:
+            xtq = NVFP4Tensor(parts[0], parts[1], BLK, torch.bfloat16, parts[2], True)
+        if ctx.have_wq_N:
+            wq_N = NVFP4Tensor(parts[-3], parts[-2], BLK, w.dtype, parts[-1], True)
         x_sharded, y_sharded = ctx.sharded[0], ctx.sharded[1]
         gy2 = gy.reshape(-1, w.shape[0])
         # a gradient split along N draws the stochastic-rounding bits of its place in the whole tensor:
@@ -335,13 +338,9 @@ class FP4Linear(nn.Module):
         if x.is_cuda and torch.is_autocast_enabled("cuda"):
             x = x.to(torch.get_autocast_dtype("cuda"))       # what autocast does for nn.Linear
         wq_K, wq_N = self._cache.get(self.weight)
-        grad_on = torch.is_grad_enabled()
-        if wq_K is None and grad_on and x.requires_grad:
-            # both layouts of the weight from one read: fprop's operand now, dgrad's for the backward
-            wq_K, wq_N = quant_weight_nvfp4(self.weight.detach())
         rht_ok = amax_signs is None or _same_signs(amax_signs, self.signs)
         return FP4LinearFn.apply(x, self.weight, self.H, self.signs, wq_K, wq_N, None, (False, False), amax, rht_ok,
-                                 None, amax_out, x_quant, grad_on)
+                                 None, amax_out, x_quant, torch.is_grad_enabled())
 
     def extra_repr(self):
         return f"in_features={self.weight.shape[1]}, out_features={self.weight.shape[0]}, bias=False, nvfp4"

@@ -196,3 +196,30 @@ def test_shared_input_quantization_equals_per_layer_quantization(Q):
     with torch.no_grad():
         xq = a.quant_input(x0)
         assert xq[1] is None and torch.equal(a(x0, x_quant=xq), a(x0))
+
+
+def test_saved_tensor_hooks_see_the_quantized_weight(Q):
+    """What a forward keeps for its backward goes through autograd's saved tensors (hooks move it, checkpointing drops
+    it): under hooks that move it to the host, the device keeps the result alone."""
+    lin = Q.FP4Linear(1024, 2048)
+    x0 = torch.randn(64, 1024, device="cuda", dtype=torch.bfloat16)
+    gy = torch.ones(64, 2048, device="cuda", dtype=torch.bfloat16)
+    grads = []
+    for offload in (True, False):
+        x = x0.clone().requires_grad_(True)
+        lin.weight.grad = None
+        lin(x)                                                        # workspaces exist from here on
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        if offload:
+            with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), lambda t: t.cuda()):
+                y = lin(x)
+            assert torch.cuda.memory_allocated() - before <= y.numel() * 2 + 4096
+        else:
+            y = lin(x)
+        from nvfp4_sm120_b200 import quant
+        quant._SEED[0] = 77
+        y.backward(gy)
+        grads.append((x.grad, lin.weight.grad))
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)
