@@ -91,6 +91,7 @@ _DUAL = [True]
 # kernel against two: 16384 x 768 nearest 15.9 / 19.3, stochastic 21.3 / 24.9; 4096 x 14336 53 / 62 and 76 / 78) and is
 # level with the two at 4096 x 28672 stochastic (144 / 143), so it takes tensors up to this many elements.
 _DUAL_MAX_ELEMS = 1 << 26
+_WEIGHT_MAX_ROWS = 64 * 65535            # what nvfp4_quantize_weight_bf16 takes
 
 
 def set_dual_quant(flag: bool):
@@ -158,7 +159,8 @@ class FP4LinearFn(torch.autograd.Function):
         else:
             xq = _quant(x2, x_red, amax=None if x_amax is None else x_amax[0:1])
         own_wq_N = None
-        if wq_K is None and grad_on and ctx.needs_input_grad[0] and amax_reduce is None:
+        if (wq_K is None and grad_on and ctx.needs_input_grad[0] and amax_reduce is None
+                and w.shape[0] <= _WEIGHT_MAX_ROWS):
             # both layouts of the weight from one read: fprop's operand now, dgrad's for the backward, which keeps 0.56 B
             # per weight element until then
             wq_K, own_wq_N = quant_weight_nvfp4(w)

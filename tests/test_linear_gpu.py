@@ -223,3 +223,13 @@ def test_saved_tensor_hooks_see_the_quantized_weight(Q):
         grads.append((x.grad, lin.weight.grad))
     for a, b in zip(*grads):
         assert torch.equal(a, b)
+
+
+def test_more_output_features_than_one_read_takes(Q):
+    """The kernel for both layouts of a weight takes 64 * 65535 rows; above them the forward quantizes the one it needs."""
+    n = 64 * 65535 + 16
+    lin = Q.FP4Linear(32, n)
+    x = torch.randn(16, 32, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    y = lin(x)
+    with torch.no_grad():
+        assert torch.equal(y, lin(x))
