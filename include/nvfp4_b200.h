@@ -218,6 +218,15 @@ int nvfp4_quantize_static_bf16(const void* x, int64_t rows, int64_t cols, int64_
 int nvfp4_quantize_static_status(int32_t* host_out, int clear, void* stream);
 
 /*
+ * Error word of the quantizer kernels that have no workspace -- everything that writes a transposed or a dual layout or
+ * a weight, the maxima after a transform along the rows, and row-wise quantization with the maximum given -- on the
+ * current device, copied to *host_out (HOST pointer): 0, or 2 = a bounded wait for a copy gave up (the outputs of that
+ * call are then undefined; the call itself has long returned NVFP4_OK).  Sticky until read with clear != 0.  Waits for
+ * `stream`; not for use during its capture.  No counterpart in the reference.
+ */
+int nvfp4_quantize_wait_status(int32_t* host_out, int clear, void* stream);
+
+/*
  * Block-scaled FP4 GEMM  D[M, N] = (A . sfA) (B . sfB)^T * (*a_pts) * (*b_pts)
  * with fp32 accumulation on the tcgen05 tensor cores.
  *   a_q [M, K/2], b_q [N, K/2]: packed E2M1, both K-major; a_sf, b_sf: swizzled E4M3 scales;
@@ -360,11 +369,12 @@ int nvfp4_rotary_bf16(const void* q, void* q_out, int q_heads, const void* k, vo
 /*
  * Test hooks of the bounded waits, process-wide, for the launches that follow.  Every spin inside
  * the kernels (grid barrier, mbarrier) gives up after a time limit, records a code (workspace word
- * 4 / the static error word for the quantizer, *status for the GEMM) and lets the kernel drain and
+ * 4 / the static error word / nvfp4_quantize_wait_status for the quantizers, *status for the GEMM) and lets the kernel drain and
  * return; these hooks let a test make that happen in a millisecond instead of never:
  *   wait_limit_ns                    the limit (0 = the default, 2 s)
  *   quantizer_extra_arrivals         the quantizer's grid barrier expects this many arrivals more
- *                                    than the grid has CTAs, so it can only run out (code 1)
+ *                                    than the grid has CTAs, so it can only run out (code 1); the
+ *                                    kernels without a workspace expect them beside every copy (code 2)
  *   gemm_drop_first_scale_arrival    != 0: the MMA issuer waits for an arrival that never comes, so the
  *                                    MMA issuer's first wait runs out (code 2) and every role leaves
  * nvfp4_test_hooks(0, 0, 0) restores normal operation.  No GPU fault, trap or endless loop is

@@ -46,6 +46,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Bounded wait for the copies of an mbarrier phase; false when it gave up.
+__device__ __forceinline__ bool wait_copy(uint32_t bar, uint32_t parity, unsigned long long limit_ns) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const unsigned long long t0 = global_ns();
+  while (!mbar_try_wait(bar, parity))
+    if (global_ns() - t0 > limit_ns) return false;
+  return true;
+}
+// nvfp4_test_hooks as it stands: the limit of the next launches' waits, and whether a wait for a copy is to run out
+unsigned long long hook_wait_limit_ns();
+uint32_t hook_extra_arrivals();
+// Error word of the kernels of a source file that have no workspace (one per device; nvfp4_quantize_wait_status reads
+// them): 2 = a copy never landed.
+static __device__ int g_wait_error;
+
 struct Scale {
   float pts, inv_pts, c;     // c ~ 1 / (6 pts), only used for the checked shortcut
 };

@@ -58,7 +58,17 @@ struct Params {
   uint8_t* q_c;
   uint8_t* sf_c;
   float* pts_c;
+  unsigned long long wait_limit_ns;
+  uint32_t extra_arrivals;       // test hook (normally 0): what the barriers of the copies expect beside the copies
 };
+
+// A CTA gives up at its tile i: records that, and leaves the copies of this tile and those already on their way behind it
+// (`slots` of them at most) a bounded time to land before its shared memory goes away.
+__device__ __forceinline__ void give_up(uint32_t bars, uint32_t slots, uint32_t i, uint32_t my_tiles, unsigned long long limit_ns) {
+  if (threadIdx.x != 0) return;
+  atomicCAS(&fused::g_wait_error, 0, 2);
+  for (uint32_t j = i; j < my_tiles && j < i + slots; ++j) fused::wait_copy(bars + 8u * (j % slots), (j / slots) & 1u, limit_ns);
+}
 
 __device__ __forceinline__ void tma_half_load(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
@@ -119,7 +129,8 @@ quant_dual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     tma_half_load(dst + kHalfBytes, &map_x, (int)(c0 + 64), (int)r0, bar);
   };
   if (tid == 0) {
-    for (int s = 0; s < kSlots; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8u * s));
+    for (int s = 0; s < kSlots; ++s)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 8u * s), "r"(1u + p.extra_arrivals));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *gave_up = 0;
     for (uint32_t i = 0; i < (uint32_t)kSlots && i < my_tiles; ++i) fetch(i);
@@ -146,13 +157,8 @@ quant_dual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   for (uint32_t i = 0; i < my_tiles; ++i) {
     int64_t r0, c0;
     locate(i, r0, c0);
-    const uint32_t slot_off = (i % kSlots) * kSlotBytes, bar = bars + 8u * (i % kSlots), parity = (i / kSlots) & 1u;
-    if (!fused::mbar_try_wait(bar, parity)) {
-      const unsigned long long t0 = fused::global_ns();
-      while (!fused::mbar_try_wait(bar, parity)) {
-        if (fused::global_ns() - t0 > fused::kWaitLimitNs) { *gave_up = 1; break; }
-      }
-    }
+    const uint32_t slot_off = (i % kSlots) * kSlotBytes, bar = bars + 8u * (i % kSlots);
+    if (!fused::wait_copy(bar, (i / kSlots) & 1u, p.wait_limit_ns)) *gave_up = 1;
     const uint8_t* slot = smem + slot_off;
     uint8_t* out = smem + kSlots * kSlotBytes + (i & 1u) * kOutBytes;
     uint8_t* out_sf = out + kTile * kOutPitch;
@@ -243,7 +249,10 @@ quant_dual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       }
     }
     __syncthreads();                                                     // the slot is read, the output collected
-    if (*gave_up != 0) return;
+    if (*gave_up != 0) {                                                 // nothing of this tile's transposed output is written
+      give_up(bars, kSlots, i, my_tiles, p.wait_limit_ns);
+      return;
+    }
     if (tid == 0 && i + kSlots < my_tiles) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // generic reads before the async write
       fetch(i + kSlots);
@@ -290,7 +299,8 @@ __device__ __forceinline__ float warp_max(float v) {
 template <bool BOTH>
 __global__ void __launch_bounds__(kThreads, 2)
 amax_tiles_kernel(const __grid_constant__ CUtensorMap map_x, uint32_t ntc, uint32_t ntiles,
-                  const float* __restrict__ signs16, float* __restrict__ out) {
+                  const float* __restrict__ signs16, float* __restrict__ out, unsigned long long wait_limit_ns,
+                  uint32_t extra_arrivals) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = fused::smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -308,7 +318,8 @@ amax_tiles_kernel(const __grid_constant__ CUtensorMap map_x, uint32_t ntc, uint3
     tma_half_load(dst + kHalfBytes, &map_x, (int)(ct * kTile + 64), (int)(rt * kTile), bar);
   };
   if (tid == 0) {
-    for (int s = 0; s < kMaxSlots; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8u * s));
+    for (int s = 0; s < kMaxSlots; ++s)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 8u * s), "r"(1u + extra_arrivals));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *gave_up = 0;
     for (uint32_t i = 0; i < (uint32_t)kMaxSlots && i < my_tiles; ++i) fetch(i);
@@ -319,13 +330,8 @@ amax_tiles_kernel(const __grid_constant__ CUtensorMap map_x, uint32_t ntc, uint3
   uint32_t mp = 0u;                                // both 16-bit halves carry a running maximum of bf16 magnitudes
   const uint32_t half = warp & 1u, rb = warp >> 1;
   for (uint32_t i = 0; i < my_tiles; ++i) {
-    const uint32_t slot = (i % kMaxSlots) * kSlotBytes, bar = bars + 8u * (i % kMaxSlots), parity = (i / kMaxSlots) & 1u;
-    if (!fused::mbar_try_wait(bar, parity)) {
-      const unsigned long long t0 = fused::global_ns();
-      while (!fused::mbar_try_wait(bar, parity)) {
-        if (fused::global_ns() - t0 > fused::kWaitLimitNs) { *gave_up = 1; break; }
-      }
-    }
+    const uint32_t slot = (i % kMaxSlots) * kSlotBytes, bar = bars + 8u * (i % kMaxSlots);
+    if (!fused::wait_copy(bar, (i / kMaxSlots) & 1u, wait_limit_ns)) *gave_up = 1;
     const uint32_t addr = fused::smem_u32(smem) + slot + half * kHalfBytes + rb * 2048u + lane * 4u;
     float v0[16], v1[16];
 #pragma unroll
@@ -350,7 +356,10 @@ amax_tiles_kernel(const __grid_constant__ CUtensorMap map_x, uint32_t ntc, uint3
     }
     m = fmaxf(m, fmaxf(fused::max_abs16(v0), fused::max_abs16(v1)));
     __syncthreads();                                                      // the slot is read
-    if (*gave_up != 0) break;
+    if (*gave_up != 0) {                                                  // no maximum of a part of the tensor
+      give_up(bars, kMaxSlots, i, my_tiles, wait_limit_ns);
+      return;
+    }
     if (tid == 0 && i + kMaxSlots < my_tiles) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");        // generic reads before the async write
       fetch(i + kMaxSlots);
@@ -442,8 +451,10 @@ int launch_amax(const void* x, int64_t rows, int64_t cols, int64_t ld, const flo
   const int64_t ntc = (cols + kTile - 1) / kTile, ntiles = ntc * ((rows + kTile - 1) / kTile);
   if (ntiles >= (1ll << 31)) return NVFP4_E_LIMIT;
   const uint32_t grid = ntiles < 2 * sms ? (uint32_t)ntiles : 2u * (uint32_t)sms;
-  if (both) amax_tiles_kernel<true><<<grid, kThreads, kMaxSmemBytes, stream>>>(map, (uint32_t)ntc, (uint32_t)ntiles, signs16, out);
-  else amax_tiles_kernel<false><<<grid, kThreads, kMaxSmemBytes, stream>>>(map, (uint32_t)ntc, (uint32_t)ntiles, signs16, out);
+  const unsigned long long limit = fused::hook_wait_limit_ns();
+  const uint32_t extra = fused::hook_extra_arrivals(), nc = (uint32_t)ntc, nt = (uint32_t)ntiles;
+  if (both) amax_tiles_kernel<true><<<grid, kThreads, kMaxSmemBytes, stream>>>(map, nc, nt, signs16, out, limit, extra);
+  else amax_tiles_kernel<false><<<grid, kThreads, kMaxSmemBytes, stream>>>(map, nc, nt, signs16, out, limit, extra);
   return cudaGetLastError() == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
 }
 
@@ -478,6 +489,8 @@ int launch(const void* x, int64_t rows, int64_t cols, int64_t ld, int rows_mode,
   p.pitch_r = counters4[0]; p.base_r = counters4[1]; p.pitch_c = counters4[2]; p.base_c = counters4[3];
   p.q_r = q_r; p.sf_r = sf_r; p.pts_r = pts_r;
   p.q_c = q_c; p.sf_c = sf_c; p.pts_c = pts_c;
+  p.wait_limit_ns = fused::hook_wait_limit_ns();
+  p.extra_arrivals = fused::hook_extra_arrivals();
   const uint32_t grid = p.nunits < 2u * (uint32_t)sms ? p.nunits : 2u * (uint32_t)sms;      // two resident CTAs per SM
   void* args[] = {&map, &p};
   if (cudaLaunchKernel(kernel_fn(rows_mode, sr_c, signs16 != nullptr), dim3(grid), dim3(kThreads), args, kSmemBytes,
@@ -490,3 +503,24 @@ int launch(const void* x, int64_t rows, int64_t cols, int64_t ld, int rows_mode,
 
 }  // namespace dual
 }  // namespace nvfp4
+
+namespace nvfp4 { namespace tiled { int wait_error_address(void** out); }}
+
+extern "C" int nvfp4_quantize_wait_status(int32_t* host_out, int clear, void* stream_) {
+  if (host_out == nullptr) return NVFP4_E_NULL;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  void* word[2] = {nullptr, nullptr};
+  int32_t got[2] = {0, 0};
+  bool ok = cudaGetSymbolAddress(&word[0], nvfp4::fused::g_wait_error) == cudaSuccess &&
+            nvfp4::tiled::wait_error_address(&word[1]) == NVFP4_OK;
+  for (int i = 0; i < 2 && ok; ++i) {
+    ok = cudaMemcpyAsync(&got[i], word[i], sizeof(int32_t), cudaMemcpyDeviceToHost, stream) == cudaSuccess;
+    if (ok && clear) ok = cudaMemsetAsync(word[i], 0, sizeof(int32_t), stream) == cudaSuccess;
+  }
+  if (!ok || cudaStreamSynchronize(stream) != cudaSuccess) {
+    cudaGetLastError();
+    return NVFP4_E_LAUNCH;
+  }
+  *host_out = got[0] != 0 ? got[0] : got[1];
+  return NVFP4_OK;
+}

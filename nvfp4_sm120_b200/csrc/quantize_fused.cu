@@ -350,6 +350,18 @@ DeviceInfo g_info[kMaxDevices];
 std::atomic<unsigned long long> g_wait_ns{0};
 std::atomic<unsigned int> g_extra_arrivals{0};
 
+}  // namespace
+
+namespace nvfp4 { namespace fused {
+unsigned long long hook_wait_limit_ns() {
+  const unsigned long long ns = g_wait_ns.load(std::memory_order_relaxed);
+  return ns != 0 ? ns : kWaitLimitNs;
+}
+uint32_t hook_extra_arrivals() { return g_extra_arrivals.load(std::memory_order_relaxed); }
+}}
+
+namespace {
+
 const void* fused_fn(bool sr, bool rht, bool known) {
 #define NVFP4_FUSED_FN(K_, T_, B_) \
   (sr ? (rht ? (const void*)quant_fused_kernel<true, true, K_, T_, B_> : (const void*)quant_fused_kernel<true, false, K_, T_, B_>) \
@@ -395,8 +407,7 @@ int device_info(DeviceInfo& out) {
 namespace nvfp4 { namespace tiled {
 int launch(const void* x, int64_t rows, int64_t cols, int64_t ld, int mode, int rht, const float* signs16,
            uint64_t seed, uint64_t offset, uint8_t* qdata, uint8_t* scales, float* pts_out, void* workspace,
-           const float* amax_in, unsigned long long wait_limit_ns, uint32_t extra_arrivals, uint64_t counter_pitch,
-           uint64_t counter_base, cudaStream_t stream);
+           const float* amax_in, uint64_t counter_pitch, uint64_t counter_base, cudaStream_t stream);
 }}
 
 static int launch_fused(const void* x, int64_t rows, int64_t cols, int64_t ld, int mode, int rht,
@@ -415,8 +426,7 @@ static int launch_fused(const void* x, int64_t rows, int64_t cols, int64_t ld, i
   const bool use_tiled = (force_tiled < 0 ? amax_in != nullptr : force_tiled != 0) || !whole;
   if (use_tiled)
     return nvfp4::tiled::launch(x, rows, cols, ld, mode, rht, signs16, seed, offset, qdata, scales, pts_out, workspace,
-                                amax_in, g_wait_ns.load(std::memory_order_relaxed),
-                                g_extra_arrivals.load(std::memory_order_relaxed), counter_pitch, counter_base, stream);
+                                amax_in, counter_pitch, counter_base, stream);
   DeviceInfo info;
   const int irc = device_info(info);
   if (irc != NVFP4_OK) return irc;
@@ -441,9 +451,8 @@ static int launch_fused(const void* x, int64_t rows, int64_t cols, int64_t ld, i
     keys.k[r][0] = (uint32_t)seed + (uint32_t)r * 0x9E3779B9u;
     keys.k[r][1] = (uint32_t)(seed >> 32) + (uint32_t)r * 0xBB67AE85u;
   }
-  unsigned long long wait_ns = g_wait_ns.load(std::memory_order_relaxed);
-  if (wait_ns == 0) wait_ns = kWaitLimitNs;
-  uint32_t extra = g_extra_arrivals.load(std::memory_order_relaxed);
+  unsigned long long wait_ns = hook_wait_limit_ns();
+  uint32_t extra = hook_extra_arrivals();
   void* args[] = {&xp, &rows32, &bpr, &ld, &fd, &signs16, &keys, &offset, &qdata, &scales, &pts_out, &ws, &per,
                   &contiguous, &amax_in, &wait_ns, &extra};
   const cudaError_t e = known ? cudaLaunchKernel(fn, dim3(grid), dim3(kThreadsKnown), args, kSmemBytes, stream)

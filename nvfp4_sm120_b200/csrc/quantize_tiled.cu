@@ -61,7 +61,8 @@ struct Params {
   Workspace* ws;
   const float* amax_in;
   unsigned long long wait_limit_ns;
-  uint32_t extra_arrivals;       // test hook: surplus arrivals the grid barrier expects (normally 0)
+  uint32_t extra_arrivals;       // test hook: surplus arrivals the grid barrier expects (normally 0), with the maximum
+                                 // given the barriers of the copies
 };
 
 __device__ __forceinline__ void tma_tile_load(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
@@ -144,7 +145,7 @@ quant_tiled_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
 
   if (tid == 0) {
     for (uint32_t b = 0; b < 2u * kSlots; ++b) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8u * b));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 8u * b), "r"(KNOWN ? 1u + p.extra_arrivals : 1u));
       asm volatile("st.shared.u32 [%0], %1;" ::"r"(counts + 4u * b), "r"(0u) : "memory");
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -213,7 +214,10 @@ quant_tiled_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
   auto fail = [&](int code) {
     *cta_abort = 1;
     if (p.ws != nullptr) p.ws->error = code;
+    else atomicCAS(&g_wait_error, 0, code);
   };
+  // a CTA that gives up leaves copies in flight time to land before its shared memory goes away
+  auto leave_copies_time = [&]() { if (tih == 0) __nanosleep(50000); };
 
   if (tih == 0) {
     const uint32_t n0 = min(np, (uint32_t)kSlots);
@@ -297,7 +301,7 @@ quant_tiled_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
       }
     }
     __syncthreads();
-    if (*cta_abort != 0) return;                  // every copy of phase 1 has landed or been given up on
+    if (*cta_abort != 0) { leave_copies_time(); return; }
     if (stamper) p.ws->after[2] = (unsigned int)(global_ns() - t_start);
     amax = red[0];
   } else {
@@ -379,7 +383,7 @@ quant_tiled_kernel(const __grid_constant__ CUtensorMap map_x, const Params p) {
     const uint16_t* tp = tab;
     uint32_t s = first_fetch % kSlots, par = (first_fetch / kSlots) & 1u;
     for (uint32_t q = 0; q < head; ++q) {
-      if (!wait_phase(full0 + 8u * s, par, cta_abort, p.wait_limit_ns)) { fail(kErrCopy); break; }
+      if (!wait_phase(full0 + 8u * s, par, cta_abort, p.wait_limit_ns)) { fail(kErrCopy); leave_copies_time(); break; }
       quantize_pair(ring + s * kPairBytes, 2u * q, tp, cur);
       tp += 2 * kHalfThreads;
       const uint32_t nq = q + kSlots;                       // the head pair this slot takes next
@@ -454,13 +458,16 @@ int device_info(DeviceInfo& out) {
 }
 }  // namespace
 
+int wait_error_address(void** out) {
+  return cudaGetSymbolAddress(out, g_wait_error) == cudaSuccess ? NVFP4_OK : NVFP4_E_LAUNCH;
+}
+
 // amax_in == nullptr: the two-phase kernel (cooperative launch: its grid barrier needs every CTA
 // resident) with the caller's workspace; otherwise one quantize pass with the given maximum, a plain
 // launch.  Arguments have been validated by the caller (quantize_fused.cu).
 int launch(const void* x, int64_t rows, int64_t cols, int64_t ld, int mode, int rht, const float* signs16,
            uint64_t seed, uint64_t offset, uint8_t* qdata, uint8_t* scales, float* pts_out, void* workspace,
-           const float* amax_in, unsigned long long wait_limit_ns, uint32_t extra_arrivals, uint64_t counter_pitch,
-           uint64_t counter_base, cudaStream_t stream) {
+           const float* amax_in, uint64_t counter_pitch, uint64_t counter_base, cudaStream_t stream) {
   DeviceInfo info;
   const int irc = device_info(info);
   if (irc != NVFP4_OK) return irc;
@@ -500,8 +507,8 @@ int launch(const void* x, int64_t rows, int64_t cols, int64_t ld, int mode, int 
   p.pts_out = pts_out;
   p.ws = static_cast<Workspace*>(workspace);
   p.amax_in = amax_in;
-  p.wait_limit_ns = wait_limit_ns != 0 ? wait_limit_ns : kWaitLimitNs;
-  p.extra_arrivals = extra_arrivals;
+  p.wait_limit_ns = hook_wait_limit_ns();
+  p.extra_arrivals = hook_extra_arrivals();
   uint32_t grid = (uint32_t)(known ? info.sm_count : (info.coop_ctas < info.sm_count ? info.coop_ctas : info.sm_count));
   const uint32_t want = (p.ntiles + 1u) / 2u;             // a tile per half CTA before more CTAs are used
   if (grid > want) grid = want;

@@ -2,6 +2,7 @@
 (nvfp4_gemm.py:30-48, nvfp4_cuda.py:158-187) on top of the sm_100a kernels."""
 from __future__ import annotations
 
+import ctypes
 import math
 
 import torch
@@ -57,10 +58,17 @@ def _workspace(device):
 
 
 def fused_error(device=None) -> int:
-    """Sticky error word of the single-launch quantizer's workspace on the current stream
-    (0 = none).  Reading it synchronises."""
-    ws = _lib.host().workspace_if_any(_device_index(device))
-    return 0 if ws is None else int(ws[4].item())
+    """Sticky error word of the quantizers (0 = none): the single-launch quantizer's workspace on the current stream, then
+    the word that the kernels without a workspace share on the device.  Reading it synchronises."""
+    index = _device_index(device)
+    ws = _lib.host().workspace_if_any(index)
+    code = 0 if ws is None else int(ws[4].item())
+    if code == 0:
+        word = ctypes.c_int32(0)
+        with torch.cuda.device(index):
+            _lib.check(_lib.lib().nvfp4_quantize_wait_status(ctypes.byref(word), 0, _stream(index)), "nvfp4_quantize_wait_status")
+        code = word.value
+    return code
 
 
 def _stream(device=None):
@@ -95,7 +103,8 @@ def quant_nvfp4(t, stochastic=False, rht=False, H=None, signs=None, seed=None, *
             _SEED[0] += 1
     _check_h(H)
     q, s, pts = _lib.host().quantize(t, bool(stochastic), bool(rht), signs, int(seed) & _M64, bool(transpose), amax,
-                                     int(philox_offset) & _M64, bool(fused), [] if counter is None else [int(v) & _M64 for v in counter[:2]])
+                                     int(philox_offset) & _M64, bool(fused),
+                                     [] if counter is None else [int(v) & _M64 for v in counter[:2]])
     return NVFP4Tensor(q, s, BLK, t.dtype, pts, True)
 
 

@@ -86,6 +86,43 @@ def test_static_entry_point_reports_a_give_up(L):
     assert L.nvfp4_quantize_static_status(None, 0, None) == -1
 
 
+def _wait_status(L, clear):
+    out = ctypes.c_int32(-77)
+    assert L.nvfp4_quantize_wait_status(ctypes.byref(out), int(clear), torch.cuda.current_stream().cuda_stream) == 0
+    return out.value
+
+
+@pytest.mark.parametrize("shape", [(512, 768), (6144, 4096)])      # fewer tiles than CTAs; more tiles than slots in each
+@pytest.mark.parametrize("call", ["both maxima", "maximum", "dual", "transposed", "weight", "row-wise"])
+def test_copy_waits_of_the_kernels_without_a_workspace(L, call, shape):
+    """Every kernel that waits for its tiles: the barriers expect one arrival too many, the launch returns, the word says
+    so, and the next call is bit-exact."""
+    import nvfp4_sm120_b200 as Q
+    from nvfp4_sm120_b200 import quant
+    x = O.synthetic_tensor(*shape, 45).cuda()
+    signs = O.signs_from_seed(4).cuda()
+    a = x.abs().max().float().reshape(1)
+    parts = lambda *qs: [p for q in qs for p in (q.qdata, q.scale.view(torch.uint8), q.per_tensor_scale)]
+    run = {"both maxima": lambda: [quant.tensor_amax_both(x, signs)],
+           "maximum": lambda: [quant.tensor_amax(x, True, signs, transpose=True)],
+           "dual": lambda: parts(*Q.quant_dual_nvfp4(x, signs, a, a, True, True, 1, 2)),
+           "transposed": lambda: parts(Q.quant_nvfp4(x, amax=a, transpose=True)),
+           "weight": lambda: parts(*Q.quant_weight_nvfp4(x, amax=a)),
+           "row-wise": lambda: parts(Q.quant_nvfp4(x, amax=a))}[call]
+    _wait_status(L, clear=True)
+    want = run()
+    assert _wait_status(L, clear=False) == 0
+    L.nvfp4_test_hooks(LIMIT_NS, 1, 0)
+    run()
+    torch.cuda.synchronize()
+    L.nvfp4_test_hooks(0, 0, 0)
+    assert _wait_status(L, clear=False) == quant.fused_error() == 2
+    assert _wait_status(L, clear=True) == 2 and _wait_status(L, clear=False) == 0
+    for u, v in zip(run(), want):
+        assert torch.equal(u, v)
+    assert _wait_status(L, clear=False) == quant.fused_error() == 0
+
+
 @pytest.mark.parametrize("mode", [1, 2])
 def test_gemm_wait_gives_up_reports_and_recovers(L, mode):
     """mode 1: one-CTA kernel, mode 2: persistent pair kernel.  The scale-factor warps never announce
