@@ -99,6 +99,19 @@ auto& g_workspaces = *new std::unordered_map<Key, at::Tensor, KeyHash>();
 auto& g_status = *new std::unordered_map<int, at::Tensor>();
 auto& g_ones = *new std::unordered_map<int, at::Tensor>();
 
+// The entry of `key`, made by `make` if there is none.  The lock is not held while it is made: a dispatch mode may run Python
+// there, which can give up the GIL or come back in here.  Of two tensors made at once the first one in stays.
+template <class Map, class Make> at::Tensor find_or_make(Map& map, const typename Map::key_type& key, Make make) {
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    const auto it = map.find(key);
+    if (it != map.end()) return it->second;
+  }
+  at::Tensor made = make();
+  std::lock_guard<std::mutex> lock(g_mutex);
+  return map.emplace(key, std::move(made)).first->second;
+}
+
 at::TensorOptions on(c10::Device dev, at::ScalarType t) { return at::TensorOptions().device(dev).dtype(t); }
 
 // 64-byte scratch of the single-launch quantizer, zeroed once, one per (device, stream): every launch leaves it ready
@@ -106,10 +119,7 @@ at::TensorOptions on(c10::Device dev, at::ScalarType t) { return at::TensorOptio
 at::Tensor workspace(int device) {
   const c10::Device dev(c10::kCUDA, (c10::DeviceIndex)device);
   const Key key{device, stream_of(dev)};
-  std::lock_guard<std::mutex> lock(g_mutex);
-  auto it = g_workspaces.find(key);
-  if (it == g_workspaces.end()) it = g_workspaces.emplace(key, at::zeros({16}, on(dev, at::kInt))).first;
-  return it->second;
+  return find_or_make(g_workspaces, key, [&] { return at::zeros({16}, on(dev, at::kInt)); });
 }
 // the workspace of the current stream if there is one yet
 OptTensor workspace_if_any(int device) {
@@ -119,20 +129,12 @@ OptTensor workspace_if_any(int device) {
   return it == g_workspaces.end() ? OptTensor() : OptTensor(it->second);
 }
 at::Tensor status_word(int device) {
-  std::lock_guard<std::mutex> lock(g_mutex);
-  auto it = g_status.find(device);
-  if (it == g_status.end())
-    it = g_status.emplace(device, at::zeros({1}, on(c10::Device(c10::kCUDA, (c10::DeviceIndex)device), at::kInt))).first;
-  return it->second;
+  return find_or_make(g_status, device,
+                      [&] { return at::zeros({1}, on(c10::Device(c10::kCUDA, (c10::DeviceIndex)device), at::kInt)); });
 }
 
 at::Tensor signs_on(const OptTensor& signs, c10::Device dev) {
-  if (!signs.has_value()) {
-    std::lock_guard<std::mutex> lock(g_mutex);
-    auto it = g_ones.find(dev.index());
-    if (it == g_ones.end()) it = g_ones.emplace(dev.index(), at::ones({16}, on(dev, at::kFloat))).first;
-    return it->second;
-  }
+  if (!signs.has_value()) return find_or_make(g_ones, dev.index(), [&] { return at::ones({16}, on(dev, at::kFloat)); });
   at::Tensor s = *signs;
   if (s.device() != dev || s.scalar_type() != at::kFloat) s = s.to(dev, at::kFloat);
   s = s.contiguous();

@@ -271,3 +271,29 @@ def test_offsets_and_counters_are_taken_modulo_2_64(Q):
         for a, b in zip(Q.quant_dual_nvfp4(x, signs, None, None, True, True, 1, 2, philox_offset=offset, counters=(4, -1, 2, 0)),
                         Q.quant_dual_nvfp4(x, signs, None, None, True, True, 1, 2, philox_offset=top, counters=(4, top, 2, 0))):
             assert same(a, b)
+
+
+def test_a_dispatch_mode_may_come_back_while_scratch_is_made(Q):
+    """The scratch words are made through torch's dispatcher: a mode that quantizes there itself does not block."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from nvfp4_sm120_b200 import quant
+    x = torch.randn(32, 64, device="cuda").to(torch.bfloat16)
+    want = Q.quant_nvfp4(x)
+
+    class Again(TorchDispatchMode):
+        inner = None
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            if self.inner is None:
+                self.inner = 0
+                self.inner = quant._workspace(x.device)
+            return func(*args, **(kwargs or {}))
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        with Again() as mode:
+            ws = quant._workspace(x.device)
+        assert ws.data_ptr() == mode.inner.data_ptr() == quant._workspace(x.device).data_ptr()
+        got = Q.quant_nvfp4(x)
+        torch.cuda.current_stream().synchronize()
+    assert torch.equal(got.qdata, want.qdata)
