@@ -116,8 +116,12 @@ def host():
         import importlib.util
         lib()
         spec = importlib.util.spec_from_file_location("_host", HOST_PATH)
-        module = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(module)
+        try:
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+        except ImportError as e:
+            raise NVFP4Error(f"{HOST_PATH} does not load (built against another torch?): build it again with "
+                             "`python -m nvfp4_sm120_b200.build`") from e
         module.init(LIB_PATH, check, cuda_device_of)
         _host = module
     return _host

@@ -13,6 +13,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 LIB = os.path.join(PKG, "libnvfp4_b200.so")
 HOST = os.path.join(PKG, "_host.so")               # native host side of the Python entry points (csrc/host)
+HOST_STAMP = os.path.join(PKG, "_host.torch")      # what it was built against
 CLI = os.path.join(PKG, "nvfp4_gemm_cli")          # stand-alone C driver of the ABI (csrc/tools)
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared", "--threads", "4"]
@@ -28,8 +29,17 @@ def _deps():
         glob.glob(os.path.join(PKG, "csrc", "host", "*.cpp"))
 
 
+def torch_build():
+    """The torch and the Python that _host.so is bound to: it loads under no other."""
+    import sysconfig
+    from importlib import metadata
+    return f"torch {metadata.version('torch')} {sysconfig.get_config_var('SOABI')}"
+
+
 def up_to_date():
-    if not all(os.path.exists(p) for p in (LIB, CLI, HOST)):
+    if not all(os.path.exists(p) for p in (LIB, CLI, HOST, HOST_STAMP)):
+        return False
+    if open(HOST_STAMP).read() != torch_build():
         return False
     t = min(os.path.getmtime(LIB), os.path.getmtime(HOST))
     return all(os.path.getmtime(p) <= t for p in _deps())
@@ -78,6 +88,8 @@ def build_host():
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("g++ failed on the host module:\n" + res.stdout + res.stderr)
+    with open(HOST_STAMP, "w") as f:
+        f.write(torch_build())
 
 
 if __name__ == "__main__":

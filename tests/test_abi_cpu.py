@@ -70,6 +70,20 @@ def test_no_cpu_path_and_loud_failure(lib, monkeypatch):
         lib.lib()
 
 
+def test_another_torch_makes_the_build_stale(lib, monkeypatch, tmp_path):
+    from nvfp4_sm120_b200 import build
+    build.build()
+    assert build.up_to_date()
+    monkeypatch.setattr(build, "torch_build", lambda: "torch 0.0 cpython-0")
+    assert not build.up_to_date()
+    stale = tmp_path / "_host.so"
+    stale.write_bytes(b"not a module")
+    monkeypatch.setattr(lib, "HOST_PATH", str(stale))
+    monkeypatch.setattr(lib, "_host", None)
+    with pytest.raises(lib.NVFP4Error, match="build it again"):
+        lib.host()
+
+
 def test_product_never_imports_the_oracle():
     pkg = os.path.join(ROOT, "nvfp4_sm120_b200")
     for dirpath, _, files in os.walk(pkg):
