@@ -282,6 +282,12 @@ int nvfp4_gemm_fp4out(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pt
 int nvfp4_gemm_set_mode(int mode);
 
 /*
+ * What nvfp4_gemm runs for a product of this size: choice3 (HOST pointer) = {1 or 2 as above, columns per tile, CTAs per
+ * tile}.  Host arithmetic only.  (nvfp4_gemm_fp4out takes 128-column tiles where this says 64 over 8 CTAs.)
+ */
+int nvfp4_gemm_choice(int64_t M, int64_t N, int64_t K, int32_t* choice3);
+
+/*
  * nvfp4_gemm with a bf16 result held in fp32: D = float(bf16(A B^T)), what nvfp4_gemm(NVFP4_OUT_BF16) and a cast give,
  * without the bf16 tensor in memory and the pass over it.  For fp32 activations: the reference's FP4Linear returns
  * its bf16 product in the activation's dtype (nvfp4_train.py:36-55).

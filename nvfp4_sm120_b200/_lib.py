@@ -67,6 +67,7 @@ _SIGS = {
                                           _c.c_void_p]),
     "nvfp4_quantize_wait_status": (_c.c_int, [_c.c_void_p, _c.c_int, _c.c_void_p]),
     "nvfp4_gemm_set_mode": (_c.c_int, [_c.c_int]),
+    "nvfp4_gemm_choice": (_c.c_int, [_c.c_int64, _c.c_int64, _c.c_int64, _c.c_void_p]),
     "nvfp4_gemm_fp4out": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p,
                                      _c.c_int64, _c.c_int64, _c.c_int64, _c.c_void_p, _c.c_void_p, _c.c_void_p,
                                      _c.c_void_p, _c.c_void_p, _c.c_void_p]),

@@ -77,6 +77,16 @@ static Choice choose(int64_t M, int64_t N, int64_t K, int forced) {
   return best;
 }
 
+extern "C" int nvfp4_gemm_choice(int64_t M, int64_t N, int64_t K, int32_t* choice3) {
+  if (choice3 == nullptr) return NVFP4_E_NULL;
+  if (M <= 0 || N <= 0 || K <= 0) return NVFP4_E_SHAPE;
+  const Choice c = choose(M, N, K, g_gemm_mode.load(std::memory_order_relaxed));
+  choice3[0] = c.pair ? 2 : 1;
+  choice3[1] = c.tile_n;
+  choice3[2] = c.splits;
+  return NVFP4_OK;
+}
+
 static int gemm_any(const uint8_t* a_q, const uint8_t* a_sf, const float* a_pts, const uint8_t* b_q,
                     const uint8_t* b_sf, const float* b_pts, void* d, int out_dtype, int64_t M, int64_t N,
                     int64_t K, int64_t ldd, uint8_t* d_sf, const float* d_amax, float* d_amax_out, int32_t* status,

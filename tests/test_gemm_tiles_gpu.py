@@ -8,6 +8,15 @@ from oracle import nvfp4_oracle as O
 
 pytestmark = pytest.mark.gpu
 
+# (tests/test_gemm_rule_cpu.py checks that these reach every choice)
+SHAPES = [
+    (512, 768, 768), (129, 72, 256), (1, 8, 32), (300, 2088, 544),       # 128 x 64 tiles, odd column halves of a scale group
+    (130, 4952, 96), (8, 11600, 2208), (1024, 4104, 992),                # 128 x 128, 128 x 256
+    (2040, 776, 3104), (1000, 2584, 2080), (3000, 3000, 800),            # pair, 256 x 128 / 192 / 256, several tiles per pair
+    (768, 768, 8192), (300, 520, 8000), (33, 72, 4128), (104, 352, 9248),    # 128 x 64 shared by 2, 4, 4, 8
+    (99, 6056, 7136), (8, 3000, 4096), (127, 2000, 8224), (64, 1096, 14336),    # 128 x 128 by 2, 4; 128 x 64 by 4; 128 x 128 by 8
+    (11, 9640, 5120), (1574, 400, 11488), (2, 2144, 11296)]              # 128 x 256 by 2, 4, 8
+
 
 @pytest.fixture(scope="module")
 def Q():
@@ -20,12 +29,7 @@ def _dequant(q):
     return O.dequant_parts(q.qdata, q.scale.view(torch.uint8), q.per_tensor_scale, rows, k).double().cuda()
 
 
-@pytest.mark.parametrize("mnk", [
-    (512, 768, 768), (129, 72, 256), (1, 8, 32),              # 128 x 64 tiles, odd column halves of a scale group
-    (300, 2088, 544), (1024, 4104, 992),                      # 128 x 128, 128 x 256
-    (2040, 776, 3104), (1000, 2584, 2080), (3000, 3000, 800),  # pair, 256 x 128 / 192 / 256, several tiles per pair
-    (300, 520, 8000), (33, 72, 4128), (8, 3000, 4096),        # shared tiles: clusters of 4, 8, 2
-    (64, 1096, 14336), (768, 768, 8192), (127, 2000, 8224)])
+@pytest.mark.parametrize("mnk", SHAPES)
 def test_rule_choices_match_the_dequantised_product(Q, mnk):
     m, n, k = mnk
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
