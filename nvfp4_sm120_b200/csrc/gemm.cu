@@ -307,7 +307,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             *reinterpret_cast<uint4*>(part + c0 + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
         }
       } else if (p.tma_store) {
-        // every MMA has finished and every TMA load has landed, so the stages are free: 32 KiB per warp
+        // every MMA has finished and every TMA load has landed, so the stages are free: 128 * TN bytes per warp
         drain_through_tma(p, &map_d, taddr, smem + (warp - 2) * (128 * TN), m0 + quad * 32, n0, 0, kTileN, alpha, lane,
                           mbits);
       } else {

@@ -4,7 +4,7 @@
 // (tile = cluster index + i * number of clusters, grouped rasterization).  The roles of a CTA:
 //   warp 0      producer: TMA tensor copies of its 128 A rows, its 128 of the 256 B rows and the scale tiles
 //               of both (cta_group::2 form, all completing on the leader's barrier; no multicast), into a
-//               ring of five stages that runs on across tiles;
+//               ring of five stages (four with 192-wide tiles) that runs on across tiles;
 //   warp 1      (leader CTA only) per K slice one barrier wait, then twelve tcgen05.cp (the scale tiles of both CTAs,
 //               shared -> tensor memory) and four tcgen05.mma cta_group::2, M 256 = 128 per CTA, N 256, K 64;
 //   warps 2-9   epilogue: tensor memory -> registers -> swizzled shared memory -> TMA store.

@@ -59,7 +59,7 @@ def test_two_cta_kernel_matches(Q, mnk, mode):
     assert ((two - ref).norm() / ref.norm()).item() < REL_TOL
     assert torch.allclose(one, two, rtol=1e-5, atol=1e-5 * ref.abs().max().item())
     assert torch.equal(two_bf, two.to(torch.bfloat16))              # same accumulation, rounded once
-    # the one-CTA fp32 result may come from the split-K path (another summation order): one bf16 ulp
+    # (one rounding of the one-CTA kernel's own fp32 sums, whose order is another one where CTAs share a tile)
     assert torch.allclose(one_bf.float(), one, rtol=2.0 ** -7, atol=1e-5 * ref.abs().max().item())
 
 
@@ -91,8 +91,8 @@ def test_many_tiles_per_cluster_and_strided_output(Q, mode):
 
 @pytest.mark.parametrize("mnk", [(256, 256, 8192), (640, 512, 16384), (768, 3072, 4096)])
 def test_split_k_small_output(Q, mnk):
-    """Weight-gradient shapes (small fp32 output, long K): K is split over several CTAs per tile that
-    add into the zeroed output; same tolerance, and the bf16 path (never split) agrees."""
+    """Weight-gradient shapes (small output, long K): the K slices of a tile are shared by a cluster of CTAs that add
+    their partial sums through shared memory, for fp32 and bf16 results alike; same tolerance."""
     m, n, k = mnk
     qa = Q.quant_nvfp4(O.synthetic_tensor(m, k, 14).cuda())
     qb = Q.quant_nvfp4(O.synthetic_tensor(n, k, 15).cuda())
