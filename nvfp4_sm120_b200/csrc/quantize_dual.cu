@@ -62,14 +62,6 @@ struct Params {
   uint32_t extra_arrivals;       // test hook (normally 0): what the barriers of the copies expect beside the copies
 };
 
-// A CTA gives up at its tile i: records that, and leaves the copies of this tile and those already on their way behind it
-// (`slots` of them at most) a bounded time to land before its shared memory goes away.
-__device__ __forceinline__ void give_up(uint32_t bars, uint32_t slots, uint32_t i, uint32_t my_tiles, unsigned long long limit_ns) {
-  if (threadIdx.x != 0) return;
-  atomicCAS(&fused::g_wait_error, 0, 2);
-  for (uint32_t j = i; j < my_tiles && j < i + slots; ++j) fused::wait_copy(bars + 8u * (j % slots), (j / slots) & 1u, limit_ns);
-}
-
 __device__ __forceinline__ void tma_half_load(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -158,7 +150,7 @@ quant_dual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     int64_t r0, c0;
     locate(i, r0, c0);
     const uint32_t slot_off = (i % kSlots) * kSlotBytes, bar = bars + 8u * (i % kSlots);
-    if (!fused::wait_copy(bar, (i / kSlots) & 1u, p.wait_limit_ns)) *gave_up = 1;
+    if (!fused::wait_copy(bar, (i / kSlots) & 1u, p.wait_limit_ns)) { *gave_up = 1; atomicCAS(&fused::g_wait_error, 0, 2); }
     const uint8_t* slot = smem + slot_off;
     uint8_t* out = smem + kSlots * kSlotBytes + (i & 1u) * kOutBytes;
     uint8_t* out_sf = out + kTile * kOutPitch;
@@ -249,10 +241,8 @@ quant_dual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       }
     }
     __syncthreads();                                                     // the slot is read, the output collected
-    if (*gave_up != 0) {                                                 // nothing of this tile's transposed output is written
-      give_up(bars, kSlots, i, my_tiles, p.wait_limit_ns);
-      return;
-    }
+    // (every copy in flight was issued before the wait that gave up began, so it has had the limit to land)
+    if (*gave_up != 0) return;
     if (tid == 0 && i + kSlots < my_tiles) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // generic reads before the async write
       fetch(i + kSlots);
@@ -331,7 +321,7 @@ amax_tiles_kernel(const __grid_constant__ CUtensorMap map_x, uint32_t ntc, uint3
   const uint32_t half = warp & 1u, rb = warp >> 1;
   for (uint32_t i = 0; i < my_tiles; ++i) {
     const uint32_t slot = (i % kMaxSlots) * kSlotBytes, bar = bars + 8u * (i % kMaxSlots);
-    if (!fused::wait_copy(bar, (i / kMaxSlots) & 1u, wait_limit_ns)) *gave_up = 1;
+    if (!fused::wait_copy(bar, (i / kMaxSlots) & 1u, wait_limit_ns)) { *gave_up = 1; atomicCAS(&fused::g_wait_error, 0, 2); }
     const uint32_t addr = fused::smem_u32(smem) + slot + half * kHalfBytes + rb * 2048u + lane * 4u;
     float v0[16], v1[16];
 #pragma unroll
@@ -356,10 +346,7 @@ amax_tiles_kernel(const __grid_constant__ CUtensorMap map_x, uint32_t ntc, uint3
     }
     m = fmaxf(m, fmaxf(fused::max_abs16(v0), fused::max_abs16(v1)));
     __syncthreads();                                                      // the slot is read
-    if (*gave_up != 0) {                                                  // no maximum of a part of the tensor
-      give_up(bars, kMaxSlots, i, my_tiles, wait_limit_ns);
-      return;
-    }
+    if (*gave_up != 0) return;                                            // no maximum of a part of the tensor
     if (tid == 0 && i + kMaxSlots < my_tiles) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");        // generic reads before the async write
       fetch(i + kMaxSlots);
