@@ -50,7 +50,7 @@ struct Choice { bool pair; int tile_n, splits; };
 // the lines fall (us, best candidate against the 256 x 256 pair tiles): 512 x 768 x 768 4.9 / 6.8 (128 x 64), 5328 x 768 x
 // 768 6.7 / 7.2 (128 x 256), 2048 x 768 x 3072 8.6 / 9.8 (pair 256 x 128), 1000 x 2584 x 7136 17.0 / 18.6 (pair 256 x 192),
 // 256 x 1024 x 8192 8.9 / 14.9 (128 x 64, four CTAs per tile), 64 x 4096 x 14336 12.6 / 22.9 (128 x 128, four),
-// 768 x 768 x 16384 15.3 / 24.7 (128 x 64, two), 8 x 14336 x 4096 11.9 / 12.6 (128 x 256, two).
+// 768 x 768 x 16384 15.7 / 24.7 (128 x 256, four), 8 x 14336 x 4096 11.9 / 12.6 (128 x 256, two).
 static Choice choose(int64_t M, int64_t N, int64_t K, int forced) {
   struct Kind { bool pair; int tile_n; float fixed, slice, drain, sum; };
   static const Kind kinds[] = {{true, 256, 5.75f, 0.315f, 1.3f, 0.0f}, {true, 192, 5.35f, 0.31f, 0.85f, 0.0f},

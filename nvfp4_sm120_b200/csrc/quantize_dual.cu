@@ -12,15 +12,16 @@
 //                of packed fp32 instructions.  Codes and scales are collected in shared memory and leave as 64
 //                contiguous bytes per output row (two full sectors) and 1024 contiguous scale bytes.
 // A tensor of fewer tiles than the chip holds CTAs is cut finer: one CTA takes a tile's row-wise output, another its
-// transposed one (512 x 768, both stochastic: 6.0 -> 4.7 us; the whole tile per CTA wins once the grid is full).
-// What bounds it: the arithmetic pipes (about 200 instructions per block with Philox and the butterfly, half of them
-// on the half-rate ALU pipe), not memory.
+// transposed one (512 x 768, both stochastic: 6.0 -> 4.7 us when this was decided; the whole tile per CTA wins once the
+// grid is full).
+// What bounds it: instruction issue and the barrier per tile, not memory: 255 warp instructions per 32 blocks with Philox
+// and the butterfly, issue slots 64 % busy, ALU pipe 47 %, heavy FMA pipe 47 %, DRAM 34 % (4096 x 14336 transposed).
 // Measured, maxima given, HBM-cold, us (before = one 64 x 64 tile per 256-thread CTA, and for the transposed output alone
 // two columns x 64 rows per thread straight from global memory):
-//   4096 x 28672   transposed nearest 68.2 -> 49.8, RHT 74.6 -> 61.1, RHT + stochastic 87.9 -> 80; both layouts
-//                  nearest 169.6 -> 98.4, stochastic 192.5 -> 139; a weight in both layouts 123.7 -> 83.6
-//   16384 x 768    transposed RHT + stochastic 17.2 -> 13.5, both layouts stochastic 24.4 -> 20.9
-//   512 x 768      transposed RHT + stochastic 6.6 -> 4.0, both layouts stochastic 4.0 -> 4.4, a weight 3.1 -> 3.7
+//   4096 x 28672   transposed nearest 68.2 -> 49.6, RHT 74.6 -> 59.0, RHT + stochastic 87.9 -> 78.3; both layouts
+//                  nearest 169.6 -> 95.7, stochastic 192.5 -> 137.5; a weight in both layouts 123.7 -> 82.9
+//   16384 x 768    transposed RHT + stochastic 17.2 -> 13.2, both layouts stochastic 24.4 -> 20.5
+//   512 x 768      transposed RHT + stochastic 6.6 -> 3.9, both layouts stochastic 4.0 -> 4.1, a weight 3.1 -> 3.4
 // Rows and columns outside the matrix get zero scale bytes, so the padding of the scale buffers needs no clearing.
 #include <mutex>
 
@@ -273,8 +274,8 @@ quant_dual_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 // The maxima of the same tiles: after the Hadamard transform along the rows, and with BOTH the plain one too
 // (out[0] = plain, out[1] = transformed; without BOTH out[0] = transformed).  Three slots of 32 KiB per CTA, two CTAs per
 // SM: 192 KiB in flight or in work per SM, one atomic per CTA and maximum.  HBM-bound, us with the clearing of the words,
-// both maxima: 4096 x 28672 51.5 -> 42.0 (5.6 TB/s), 4096 x 14336 30.8 -> 25.1, 4096 x 4096 14.7 -> 12.7, 16384 x 768
-// 14.7 -> 11.4, 512 x 768 7.3 -> 6.4 (before: a CTA per 64 rows x 512 columns, staged through registers, thousands of CTAs).
+// both maxima: 4096 x 28672 51.5 -> 41.2 (5.7 TB/s), 4096 x 14336 30.8 -> 24.6, 4096 x 4096 14.7 -> 12.4, 16384 x 768
+// 14.7 -> 10.8, 512 x 768 7.3 -> 6.0 (before: a CTA per 64 rows x 512 columns, staged through registers, thousands of CTAs).
 // ---------------------------------------------------------------------------------------
 constexpr int kMaxSlots = 3;
 constexpr int kMaxMiscOff = kMaxSlots * kSlotBytes;

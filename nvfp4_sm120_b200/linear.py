@@ -88,8 +88,8 @@ def _take_grad_amax(gy2, signs=None):
 
 _DUAL = [True]
 # The one-read kernel wins wherever a second read, launch or maximum counts (measured on a B200, maxima given, us, one
-# kernel against two: 16384 x 768 nearest 15.9 / 19.3, stochastic 21.3 / 24.9; 4096 x 14336 53 / 62 and 76 / 78) and is
-# level with the two at 4096 x 28672 stochastic (144 / 143), so it takes tensors up to this many elements.
+# kernel against two: 16384 x 768 nearest 15.4 / 19.2, stochastic 20.5 / 24.0; 4096 x 14336 52.6 / 59.9 and 73.5 / 74.8) and is
+# level with the two at 4096 x 28672 stochastic (137.5 / 135.2), so it takes tensors up to this many elements.
 _DUAL_MAX_ELEMS = 1 << 26
 _WEIGHT_MAX_ROWS = 64 * 65535            # what nvfp4_quantize_weight_bf16 takes
 
