@@ -225,9 +225,9 @@ at::Tensor amax_both(const at::Tensor& t, const OptTensor& signs) {
   return amax_both_rows(x, signs_on(signs, x.device()));
 }
 
-// counter: empty (the tensor is whole), or pitch and base
+// shard: pitch and base number the blocks; otherwise the tensor is whole
 py::tuple quantize(const at::Tensor& t, bool stochastic, bool rht, const OptTensor& signs, uint64_t seed, bool transpose,
-                   const OptTensor& amax_in, uint64_t offset, bool fused, const std::vector<uint64_t>& counter) {
+                   const OptTensor& amax_in, uint64_t offset, bool fused, bool shard, uint64_t pitch, uint64_t base) {
   check_matrix(t);
   const c10::cuda::CUDAGuard guard(t.device());
   // fp32 without a known maximum: the rounding finds it on the way.  Row-wise the single-launch kernel needs no pass of
@@ -254,9 +254,8 @@ py::tuple quantize(const at::Tensor& t, bool stochastic, bool rht, const OptTens
     return py::make_tuple(o.q, o.s, o.p);
   }
   const at::Tensor a = known != nullptr ? *known : amax_rows(x, rht, rht ? &sg : nullptr, transpose, OptTensor());
-  const bool shard = counter.size() == 2;
   check(lib.nvfp4_quantize_shard_bf16(x.data_ptr(), rows, cols, x.stride(0), transpose, stochastic, rht, sgp, float_ptr(a),
-                                      seed, offset, shard ? counter[0] : (uint64_t)(k / 16), shard ? counter[1] : 0, o.qp(),
+                                      seed, offset, shard ? pitch : (uint64_t)(k / 16), shard ? base : 0, o.qp(),
                                       o.sp(), o.pp(), stream),
         "nvfp4_quantize_shard_bf16");
   return py::make_tuple(o.q, o.s, o.p);

@@ -102,9 +102,9 @@ def quant_nvfp4(t, stochastic=False, rht=False, H=None, signs=None, seed=None, *
         if stochastic:
             _SEED[0] += 1
     _check_h(H)
+    pitch, base = (0, 0) if counter is None else (int(counter[0]) & _M64, int(counter[1]) & _M64)
     q, s, pts = _lib.host().quantize(t, bool(stochastic), bool(rht), signs, int(seed) & _M64, bool(transpose), amax,
-                                     int(philox_offset) & _M64, bool(fused),
-                                     [] if counter is None else [int(v) & _M64 for v in counter[:2]])
+                                     int(philox_offset) & _M64, bool(fused), counter is not None, pitch, base)
     return NVFP4Tensor(q, s, BLK, t.dtype, pts, True)
 
 
